@@ -59,14 +59,28 @@ struct SoloSmem {
     uint32_t tab[H];
     uint32_t so_idx[EMAX];  // the children's ranked order: rank -> compacted index
     // the chunk's children in edge order: node, row start, and valence with
-    // the parent's chunk index in the high bits (valence < 2^kParShift)
-    uint32_t ch_c[EMAX], ch_rs[EMAX], ch_dp[EMAX];
+    // the parent's chunk index in the high bits (valence < 2^kParShift); in
+    // an unordered pass (solo_level_pass) instead the entries of each warp's
+    // rows and the queue records of the current and the next level (the
+    // first CAP of each)
+    static constexpr int CAP = EMAX / 4 < B ? EMAX / 4 : B;
+    static_assert(2 * W * 32 * 8 + 16 * CAP <= 12 * EMAX, "the level pass fits the chunk's child arrays");
+    union {
+        struct {
+            uint32_t ch_c[EMAX], ch_rs[EMAX], ch_dp[EMAX];
+        };
+        struct {
+            uint2 lbuf[2][CAP];
+            uint16_t ent[W][32 * 8];
+        };
+    };
     uint32_t wcnt[W], wdeg[W];
     uint32_t scanbuf[2][W];
     uint32_t tmp32[W + 1];
     unsigned long long tmp64[2 * W + 2];
     uint32_t m, Ec;
     uint32_t bcast[4];
+    uint32_t lcnt[3];  // level pass: children of level L at [L % 3]
 };
 
 // Chunk edge indices take kEdgeBits bits below the node in a dedup word
@@ -464,6 +478,167 @@ __device__ void solo_pass(Solo<B, EMAX>& so, uint32_t start, bool sorted, bool w
     last_start = lstart;
 }
 
+// Sets bits of *p under a predicate, without a branch around the atomic (eight
+// in a row are in flight together); the old word, or all ones when off.
+template <bool GV>
+__device__ __forceinline__ uint32_t or_if(uint32_t* p, uint32_t v, bool on)
+{
+    uint32_t old = 0xFFFFFFFFu;
+    if (GV)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t@p atom.global.or.b32 %0, [%1], %2;\n\t}"
+                     : "+r"(old)
+                     : "l"(__cvta_generic_to_global(p)), "r"(v), "r"((uint32_t)on)
+                     : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t@p atom.shared.or.b32 %0, [%1], %2;\n\t}"
+                     : "+r"(old)
+                     : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v), "r"((uint32_t)on)
+                     : "memory");
+    return old;
+}
+
+// One breadth-first pass from `start`, unordered inside a level: what a
+// start-search pass needs when its order does not matter (see solo_reorder).
+// Test-and-set of the visited bit is the whole dedup, and the group meets
+// once a level: each warp takes up to 32 parents at a time, as many as have
+// 256 entries between them, deals their entries out to its lanes in order
+// (entry e = lane + 32 u; ent[e] = parent lane << 5 | slot names its row), and
+// appends the children it marked.  A row of more than 31 entries goes alone.
+// Returns the last level's records in s.lbuf[(nlevels - 1) & 1] (those past
+// CAP in the queue).  GV: the visited bitmap is in global memory.
+template <bool GV, int B, int EMAX>
+__device__ void solo_level_pass(Solo<B, EMAX>& so, uint32_t start, uint32_t& placed, uint32_t& nlevels,
+                                uint32_t& last_start)
+{
+    using S = SoloSmem<B, EMAX>;
+    constexpr uint32_t CAP = (uint32_t)S::CAP;
+    constexpr int U = 8;
+    S& s = so.s;
+    const MatrixView& M = so.M;
+    const uint32_t n = M.n;
+    const uint2* const e2 = so.e2;
+    uint2* const q = so.q;
+    uint32_t* const vis = GV ? so.gvis : s.vis;
+    const uint32_t t = gtid<B>(), lane = t & 31u, w = t >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t words = (n + 31u) / 32u;
+    for (uint32_t i = t; i < words; i += B)
+        vis[i] = 0u;
+    gsync<B>();
+    if (t == 0) {
+        const uint32_t a = ld_ro(M.rp + start), b = ld_ro(M.rp + start + 1);
+        s.lbuf[0][0] = solo_rec(start, b - a, a);
+        so.mark(start);
+        s.lcnt[0] = 0;
+        s.lcnt[1] = 0;
+        s.lcnt[2] = 0;
+    }
+    gsync<B>();
+    uint32_t head = 0, lvl_end = 1, L = 0, slot = 0;
+    while (true) {
+        const uint2* cur = s.lbuf[L & 1u];
+        uint2* nxt = s.lbuf[(L & 1u) ^ 1u];
+        const uint32_t width = lvl_end - head;
+        // the warps' shares of the level: consecutive parents
+        const uint32_t share = (width + B / 32 - 1) / (B / 32);
+        const uint32_t bend = min(width, (w + 1) * share);
+        for (uint32_t b = w * share; b < bend;) {
+            const uint32_t i = b + lane;
+            uint2 r = make_uint2(0u, 0u);
+            if (i < bend)
+                r = i < CAP ? cur[i] : __ldcg(q + head + i);
+            const uint32_t deg = rec_deg(r);
+            uint32_t x = deg;
+#pragma unroll
+            for (uint32_t o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFull, x, o);
+                x += lane >= o ? y : 0u;
+            }
+            // the parents taken: the longest prefix of rows of at most 31
+            // entries, 32 U between them; or one longer row
+            const uint32_t bad = ~__ballot_sync(kFull, i < bend && deg < 32u && x <= 32u * U);
+            const uint32_t m = bad ? (uint32_t)__ffs(bad) - 1u : 32u;
+            const uint32_t took = max(m, 1u);
+            const uint32_t soff = x - deg, shift = r.y - soff;
+            const uint32_t E = __shfl_sync(kFull, x, (int)took - 1);
+            __syncwarp();
+            if (lane < m)
+                for (uint32_t k = 0; k < deg; ++k)
+                    s.ent[w][soff + k] = (uint16_t)lane;
+            __syncwarp();
+            for (uint32_t e0 = 0; e0 < E; e0 += 32u * U) {
+                uint2 v[U];
+                uint32_t cand = 0;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t e = e0 + 32u * u + lane;
+                    v[u] = make_uint2(0u, 0u);
+                    if (e0 + 32u * u < E) {
+                        const uint32_t j = m != 0 ? (uint32_t)s.ent[w][32u * u + lane] : 0u;
+                        const uint32_t idx = __shfl_sync(kFull, shift, (int)j) + e;
+                        const bool in = e < E && PB_CHECK(M.res, idx < M.nnz, 611);
+                        v[u] = __ldcg(e2 + (in ? idx : 0u));
+                        cand |= in ? 1u << u : 0u;
+                    }
+                }
+                uint32_t old[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t c = rec_node(v[u]);
+                    const uint32_t word = GV ? __ldcg(vis + (c >> 5)) : vis[c >> 5];
+                    if ((word >> (c & 31u)) & 1u)
+                        cand &= ~(1u << u);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t c = rec_node(v[u]), bit = 1u << (c & 31u);
+                    old[u] = or_if<GV>(vis + (c >> 5), bit, (cand >> u) & 1u) & bit;
+                }
+                // the children this warp marked, behind those of the others
+                uint32_t bal[U], tot = 0;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    bal[u] = __ballot_sync(kFull, old[u] == 0u);
+                    tot += __popc(bal[u]);
+                }
+                if (tot != 0) {
+                    uint32_t at = 0;
+                    if (lane == 0)
+                        at = atomicAdd(&s.lcnt[slot], tot);
+                    at = __shfl_sync(kFull, at, 0);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const uint32_t p = at + __popc(bal[u] & lt);
+                        if (old[u] == 0u) {
+                            if (p < CAP)
+                                nxt[p] = v[u];
+                            else if (PB_CHECK(M.res, lvl_end + p < n, 612))
+                                __stcg(q + lvl_end + p, v[u]);
+                        }
+                        at += __popc(bal[u]);
+                    }
+                }
+            }
+            b += took;
+        }
+        gsync<B>();
+        const uint32_t cnt = s.lcnt[slot];
+        slot = slot == 2 ? 0 : slot + 1;
+        // the counter of the level after next: last read before this barrier
+        if (t == 0)
+            s.lcnt[slot == 2 ? 0 : slot + 1] = 0;
+        if (cnt == 0)
+            break;
+        head = lvl_end;
+        lvl_end += cnt;
+        ++L;
+    }
+    gsync<B>();
+    placed = lvl_end;
+    nlevels = L + 1;
+    last_start = head;
+}
+
 // Full reorder of one matrix by one solo group: start search
 // (simple_peripheral.cpp:92-141), the sorted pass, reverse, bandwidth.
 // e2: the matrix's edge records; inv: n words for the inverse permutation;
@@ -498,7 +673,27 @@ __device__ void solo_reorder(SoloSmem<B, EMAX>& s, const MatrixView& M, const ui
             break;
         if (searching)
             ++passes;
-        solo_pass<B, EMAX>(so, start, !searching, !searching, opt.reverse != 0, placed, nlevels, last_start);
+        // a start-search pass has to deliver its level count and the next
+        // start, and that start -- the last node of minimal valence among the
+        // last outnodes discovered, on the last level
+        // (simple_peripheral.cpp:118-127) -- does not depend on the order
+        // when the last level has at most outnodes nodes and one of them
+        // alone has the minimal valence: the search runs unordered and is
+        // only repeated in order where that fails (never on grids; a third of
+        // the passes of random geometric graphs).  From the third pass on,
+        // which usually confirms the eccentricity, the pass of a sparse
+        // matrix is the sorted one itself: the result if it does (444 at once
+        // of 100,000 nodes: 2-D grids 12.3 ms against 14.1 with a third
+        // unordered pass, 3-D grids 15.3 / 16.6; but random geometric graphs
+        // of 11 entries a row, whose third pass confirms less often and whose
+        // sorted pass costs two unordered ones, 38.0 / 35.0).
+        const bool sorted = !searching || (passes >= 3 && opt.mode != kModeStartOnly && M.nnz <= 8ull * n);
+        if (sorted)
+            solo_pass<B, EMAX>(so, start, true, true, opt.reverse != 0, placed, nlevels, last_start);
+        else if (so.gvis)
+            solo_level_pass<true, B, EMAX>(so, start, placed, nlevels, last_start);
+        else
+            solo_level_pass<false, B, EMAX>(so, start, placed, nlevels, last_start);
         if (read_status(M.res) != 0)
             return;
         if (!searching)
@@ -511,12 +706,45 @@ __device__ void solo_reorder(SoloSmem<B, EMAX>& s, const MatrixView& M, const ui
         const uint32_t dist = nlevels - 1;
         if (dist == lastdist) {
             ecc = dist;
-            searching = false;  // the sorted pass from the same start comes next
-            continue;
+            searching = false;
+            if (sorted)
+                break;  // confirmed by the sorted pass: the result
+            continue;   // the sorted pass from the same start comes next
         }
-        if (t == 0)
-            s.bcast[0] = so.next_start(opt.outnodes, last_start);
-        gsync<B>();
+        const uint32_t width = n - last_start;
+        bool known = false;
+        if (width <= min(opt.outnodes, n - 1) && width <= (uint32_t)SoloSmem<B, EMAX>::CAP) {
+            if (t < 32) {
+                uint32_t d = kUnvisited, v = 0, same = 0;
+                for (uint32_t i = t; i < width; i += 32) {
+                    const uint2 r = sorted ? __ldcg(so.q + last_start + i) : s.lbuf[(nlevels - 1) & 1u][i];
+                    const uint32_t di = rec_deg(r);
+                    same = di < d ? 1u : same + (di == d ? 1u : 0u);
+                    if (di < d) {
+                        d = di;
+                        v = rec_node(r);
+                    }
+                }
+                const uint32_t dm = __reduce_min_sync(kFull, d);
+                const uint32_t count = __reduce_add_sync(kFull, d == dm ? same : 0u);
+                v = __shfl_sync(kFull, v, __ffs(__ballot_sync(kFull, d == dm)) - 1);
+                if (t == 0) {
+                    s.bcast[0] = v;
+                    s.bcast[1] = count;
+                }
+            }
+            gsync<B>();
+            known = s.bcast[1] == 1u;
+        }
+        if (!known) {
+            gsync<B>();
+            solo_pass<B, EMAX>(so, start, false, false, false, placed, nlevels, last_start);
+            if (read_status(M.res) != 0)
+                return;
+            if (t == 0)
+                s.bcast[0] = so.next_start(opt.outnodes, last_start);
+            gsync<B>();
+        }
         start = s.bcast[0];
         gsync<B>();
         lastdist = dist;
