@@ -1,5 +1,7 @@
-// pool_p6.cu -- batch kernels of pool shape 6: 256-thread CTAs of one group with 1024-edge chunks, three per SM
-// (the solo engine's shared memory packed to 72 KB, 80 registers).
+// pool_p6.cu -- batch kernels of pool shape 6: 256-thread CTAs of one group with 1024-edge chunks; the solo batch
+// kernel two per SM (128 registers).  What a third group adds in flight it takes from the others' share of L2 (the
+// matrices' edge records and positions are read at random): 4,096 mixed matrices 66.4 ms with three CTAs of 80
+// registers, 58.6 with two; 73.2 with one CTA of 512 threads.
 #include "pool.cuh"
 
-PBRCM_DEFINE_POOL(6, 256, 1024, 256, 1024, 3, 3)
+PBRCM_DEFINE_POOL(6, 256, 1024, 256, 1024, 3, 2)
