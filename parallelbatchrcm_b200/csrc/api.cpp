@@ -61,7 +61,6 @@ void apply_team_shape(const Context& C, Options& opt)
     opt.solo_edges = C.solo_edges;
     opt.solo_parents = C.solo_parents;
     opt.barrier = C.barrier;
-    opt.spec_from = C.spec_from;
 }
 
 void fill_result(const DevResult& r, const Options& opt, pbrcm_result* out)
@@ -123,7 +122,7 @@ int32_t Context::init(int dev)
     if (cudaMallocHost(&h_one, sizeof(uint32_t)) != cudaSuccess)
         return PBRCM_ERR_OOM;
     *h_one = 1u;
-    if (cudaMalloc(&d_res, sizeof(DevResult)) != cudaSuccess || cudaMalloc(&d_gs, kTeamParts * sizeof(GridSync)) != cudaSuccess)
+    if (cudaMalloc(&d_res, sizeof(DevResult)) != cudaSuccess || cudaMalloc(&d_gs, sizeof(GridSync)) != cudaSuccess)
         return PBRCM_ERR_OOM;
     if (cudaMallocHost(&h_res, sizeof(DevResult)) != cudaSuccess ||
         cudaMallocHost(&h_aux, 64) != cudaSuccess)
@@ -145,7 +144,6 @@ int32_t Context::init(int dev)
     solo_parents = (uint32_t)env_int("PBRCM_SOLO_PARENTS", kVariants[team_variant].block);
     solo_edges = (uint32_t)env_int("PBRCM_SOLO_EDGES", kVariants[team_variant].emax);
     barrier = (uint32_t)env_int("PBRCM_BARRIER", 0) ? 1u : 0u;
-    spec_from = (uint32_t)std::max(0, env_int("PBRCM_SPEC_FROM", 3));
     // wide, shallow graphs: PBRCM_WIDE_DIV (0: never), PBRCM_WIDE_MIN,
     // PBRCM_ENGINE=wide to run the level-synchronous engine first, =team for
     // the team engine alone
@@ -202,7 +200,7 @@ int32_t Context::init(int dev)
     solo = env_int("PBRCM_SOLO", 1) != 0;
     batch_solo_kernel = env_int("PBRCM_BATCH_SOLO_KERNEL", (int)tn.batch_kernel) != 0;
     batch_graphs = env_int("PBRCM_BATCH_GRAPHS", 1) != 0;
-    if (cudaMalloc(&d_agg, kTeamParts * team_part_bytes(maxc)) != cudaSuccess)
+    if (cudaMalloc(&d_agg, team_words_bytes(maxc)) != cudaSuccess)
         return PBRCM_ERR_OOM;
     // cluster teams of the batch path (PBRCM_BATCH_CLUSTER* override)
     // measured on the mixed 1,024-matrix batch: pairs for the 16 biggest
@@ -222,7 +220,7 @@ Context::~Context()
         cudaSetDevice(device);
     if (stream)
         cudaStreamSynchronize(stream);
-    for (void* p : {(void*)d_wide, (void*)d_pw, (void*)d_rp, (void*)d_ci, (void*)d_node, (void*)d_perm, (void*)d_rec, (void*)d_rec2, (void*)d_stage, (void*)d_hub,
+    for (void* p : {(void*)d_wide, (void*)d_pw, (void*)d_rp, (void*)d_ci, (void*)d_node, (void*)d_perm, (void*)d_rec, (void*)d_stage, (void*)d_hub,
                     (void*)d_res, (void*)d_gs, (void*)d_agg, (void*)d_jobs, (void*)d_slots, (void*)d_counter, (void*)d_bres,
                     (void*)d_arena})
         if (p)
@@ -278,8 +276,8 @@ bool Context::ensure_single(uint32_t n, uint64_t nnz, bool inputs)
 {
     if (inputs && (!grow(d_rp, cap_rp, (size_t)n + 1) || !grow(d_ci, cap_ci, (size_t)nnz)))
         return false;
-    return grow(d_node, cap_node, n) && grow(d_rec, cap_rec, n) && grow(d_rec2, cap_rec2, n) &&
-           grow(d_stage, cap_stage, 2 * std::max<uint64_t>(nnz, 1)) && grow(d_perm, cap_perm, n);
+    return grow(d_node, cap_node, n) && grow(d_rec, cap_rec, n) &&
+           grow(d_stage, cap_stage, std::max<uint64_t>(nnz, 1)) && grow(d_perm, cap_perm, n);
 }
 
 bool Context::ensure_hub(uint64_t nnz) { return grow(d_hub, cap_hub, 4 * (size_t)std::max<uint64_t>(nnz, 1)); }
@@ -382,14 +380,13 @@ int32_t Context::run_single(const uint32_t* rp, const uint32_t* ci, uint32_t n, 
         M.nnz = (uint32_t)nnz;
         M.node = d_node;
         M.rec = d_rec;
-        M.rec2 = d_rec2;
         M.stage = d_stage;
         M.perm = perm;
         M.hub = with_hub ? d_hub : nullptr;
         M.res = d_res;
         if (cudaMemsetAsync(d_res, 0, sizeof(DevResult), st) != cudaSuccess ||
-            cudaMemsetAsync(d_gs, 0, kTeamParts * sizeof(GridSync), st) != cudaSuccess ||
-            cudaMemsetAsync(d_agg, 0, kTeamParts * team_part_bytes(team_ctas), st) != cudaSuccess)
+            cudaMemsetAsync(d_gs, 0, sizeof(GridSync), st) != cudaSuccess ||
+            cudaMemsetAsync(d_agg, 0, team_words_bytes(team_ctas), st) != cudaSuccess)
             return PBRCM_ERR_CUDA;
         if (launch_validate(rp, ci, n, (uint32_t)nnz, d_res, sms, st) != cudaSuccess)
             return PBRCM_ERR_CUDA;

@@ -30,7 +30,6 @@ struct Context {
     uint32_t solo_edges = 0;    // levels at most this big run on one CTA
     uint32_t solo_parents = 0;
     uint32_t barrier = 0;       // team barrier implementation
-    uint32_t spec_from = 3;     // speculative split from this search pass on (team-dominated matrices)
     int team_maxc = 0;          // co-resident CTAs of the team kernel
     // the level-synchronous engine for wide, shallow graphs (wide.cu): a
     // first-pass level of at least max(n / wide_div, wide_min) nodes hands
@@ -72,9 +71,7 @@ struct Context {
     size_t cap_perm = 0;
     PosRec* d_rec = nullptr;
     size_t cap_rec = 0;
-    PosRec* d_rec2 = nullptr;  // queue records of the speculative ordered pass
-    size_t cap_rec2 = 0;
-    PosRec* d_stage = nullptr;  // staged children of multi-chunk team levels (2 nnz)
+    PosRec* d_stage = nullptr;  // staged children of multi-chunk team levels (nnz)
     size_t cap_stage = 0;
     uint32_t* d_hub = nullptr;
     size_t cap_hub = 0;

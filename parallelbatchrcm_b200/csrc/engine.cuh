@@ -99,14 +99,7 @@ __device__ __forceinline__ uint32_t ld_ro(const uint32_t* p) { return __ldg(p); 
 
 __device__ __forceinline__ uint4 ld_node(const NodeEntry* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
 
-// The claim word a pass uses: NodeEntry::claim (M.cf == 0) or, for the
-// speculative ordered pass that runs beside a start-search pass, the word
-// NodeEntry::inv (M.cf == 3; inv is only used after the last pass).
-__device__ __forceinline__ uint32_t* claim_ptr(const MatrixView& M, uint32_t v)
-{
-    return reinterpret_cast<uint32_t*>(M.node + v) + M.cf;
-}
-__device__ __forceinline__ uint32_t claim_of(const MatrixView& M, const uint4& nd) { return M.cf ? nd.w : nd.x; }
+__device__ __forceinline__ uint32_t* claim_ptr(const MatrixView& M, uint32_t v) { return &M.node[v].claim; }
 
 __device__ __forceinline__ void set_status(DevResult* r, uint32_t code, uint32_t where)
 {
@@ -302,7 +295,7 @@ __device__ __forceinline__ void block_reduce_sum2(unsigned long long& a, unsigne
 }
 
 // Level state of one pass, the same in every CTA of a team.
-constexpr int kTeamShared = 12;  // group-shared ints a team needs (Team::sh)
+constexpr int kTeamShared = 14;  // group-shared ints a team needs (Team::sh)
 
 struct LevelState {
     uint32_t a, b;     // frontier positions [a, b)
@@ -325,6 +318,7 @@ struct Team {
     uint32_t target;     // barriers passed so far
     uint32_t mode;       // barrier implementation (see sync)
     uint32_t epoch;      // gate epochs seen
+    uint32_t word = 0;   // level_sync barriers passed
     unsigned long long wait_ns;
     DevResult* res;
     // the thread group running this CTA's part (see gtid): its thread 0 is
@@ -411,6 +405,57 @@ struct Team {
         const int ok = s_ok && read_status(res) == 0;
         gbar();
         return ok != 0;
+    }
+
+    // The barrier of an unordered level (level_pass), in two halves so that
+    // work goes on in between: one 64-bit word gathers the arrivals, the
+    // requests for a new split and the level's totals (fields of 8, 8, 24 and
+    // 24 bits: at most 255 CTAs of at most EMAX nodes and entries each; more
+    // than that comes with a request).  The words turn by threes in gs->word,
+    // each cleared two barriers before its use.
+    __device__ __forceinline__ void level_arrive(uint32_t cnt, uint32_t esum, bool ask)
+    {
+        if (tid == 0) {
+            const unsigned long long v = 1ull << 56 | (unsigned long long)(ask ? 1u : 0u) << 48 |
+                                         (unsigned long long)(ask ? 0u : esum) << 24 | (ask ? 0u : cnt);
+            asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&gs->word[word % 3u]), "l"(v) : "memory");
+        }
+    }
+    // keep: nobody asked for a new split.  False: the team must stop.
+    __device__ bool level_wait(uint32_t where, uint32_t& all_cnt, uint32_t& all_esum, bool& keep)
+    {
+        int& s_ok = sh[(word & 1u) ? 1 : 10];
+        gbar();
+        if (tid == 0) {
+            const uint32_t st0 = read_status(res);
+            unsigned long long t0 = 0, got;
+            uint32_t spins = 0;
+            int ok = 1;
+            while (true) {
+                asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(got) : "l"(&gs->word[word % 3u]) : "memory");
+                if ((uint32_t)(got >> 56) >= expected)
+                    break;
+                if ((++spins & 31u) == 0 && !wait_check(t0, where)) {
+                    ok = 0;
+                    break;
+                }
+                if (spins > 2048)
+                    __nanosleep(128);
+            }
+            // the word after next: everyone is past its last use
+            if (rank == 0)
+                st_relaxed64(&gs->word[(word + 2u) % 3u], 0ull);
+            sh[11] = (int)(uint32_t)((got >> 48) & 0xFFu);
+            sh[12] = (int)(uint32_t)((got >> 24) & 0xFFFFFFu);
+            sh[13] = (int)(uint32_t)(got & 0xFFFFFFu);
+            s_ok = ok && st0 == 0;
+        }
+        gbar();
+        ++word;
+        keep = sh[11] == 0;
+        all_esum = (uint32_t)sh[12];
+        all_cnt = (uint32_t)sh[13];
+        return s_ok != 0;
     }
 
     // Shared by every bounded wait: false once an error is posted or the
@@ -915,7 +960,7 @@ struct Chunk {
         uint32_t pos[MAXEPT];
 #pragma unroll
         for (int r = 0; r < MAXEPT; ++r) {
-            if (!(c[r] != kUnvisited && c[r] < M.n && claim_of(M, nd[r]) == key[r]))
+            if (!(c[r] != kUnvisited && c[r] < M.n && nd[r].x == key[r]))
                 c[r] = kUnvisited;
             const uint32_t bal = __ballot_sync(kFull, c[r] != kUnvisited);
             pos[r] = __popc(bal & ((1u << lane) - 1u));
@@ -989,6 +1034,150 @@ struct Chunk {
         }
         gsync<B>();
         return Agg{Q, Qdeg};
+    }
+
+    // ---- unordered passes (level_pass) --------------------------------
+    // A list of queue entries in shared memory (node, row start, valence):
+    // two of EMAX entries, in the child arrays and in the room of the
+    // prefetched adjacency.
+    struct List {
+        uint32_t *node, *rs, *deg;
+    };
+    __device__ __forceinline__ List list(uint32_t which) const
+    {
+        return which ? List{s.pre, s.pre + EMAX, s.pre + 2 * EMAX} : List{s.ch_node, s.ch_rs, s.ch_deg};
+    }
+
+    // The next chunk's parents from entries [p, F) of a list: the longest run
+    // of at most B parents with at most EMAX edges.  Returns their number.
+    __device__ uint32_t form_list(const List& P, uint32_t p, uint32_t F)
+    {
+        const uint32_t t = gtid<B>();
+        const bool have = p + t < F;
+        const uint32_t deg = have ? P.deg[p + t] : 0u;
+        uint32_t total;
+        const uint32_t excl = block_scan1<B>(deg, total, s.scanbuf[1]);
+        uint32_t m = F - p;
+        if (m > (uint32_t)B || total > (uint32_t)EMAX)  // the same in every thread
+            m = (uint32_t)gsync_count<B>(have && excl + deg <= (uint32_t)EMAX);
+        if (t < m) {
+            s.prs[t] = P.rs[p + t];
+            s.soff[t] = excl;
+            if (t == m - 1) {
+                s.soff[m] = excl + deg;
+                s.m = m;
+                s.Ec = excl + deg;
+            }
+        }
+        gsync<B>();
+        return m;
+    }
+
+    // The columns of the chunk's edges: thread t's are t + B r.
+    __device__ __forceinline__ void load_cols(uint32_t c[MAXEPT]) const
+    {
+        const uint32_t t = gtid<B>();
+        const uint32_t m = s.m, Ec = s.Ec;
+#pragma unroll
+        for (int r = 0; r < MAXEPT; ++r) {
+            const uint32_t e = t + (uint32_t)B * r;
+            c[r] = kUnvisited;
+            if (e < Ec) {
+                uint32_t j = 0;
+#pragma unroll
+                for (uint32_t d = (uint32_t)B / 2u; d > 0; d >>= 1) {
+                    const uint32_t mid = j + d;
+                    if (mid < m && s.soff[mid] <= e)
+                        j = mid;
+                }
+                const uint32_t idx = s.prs[j] + (e - s.soff[j]);
+                if (PB_CHECK(M.res, idx < M.nnz, 152))
+                    c[r] = ld_ro(M.ci + idx);
+            }
+        }
+    }
+
+    // The unordered form of collect: those of the chunk's columns that no
+    // edge of this pass has claimed yet (claims below `first` are earlier
+    // passes'), each new node once; its claim and its node entry come with
+    // one round trip, side by side.  They go behind the C.cnt entries of
+    // list `out`, which `flush` empties first when they do not fit.
+    // counted(C) is called once their number is known, before they are
+    // listed.
+    template <typename Flush, typename Counted>
+    __device__ void claim_list(uint32_t first, const uint32_t c[MAXEPT], const List& out, Agg& C, Flush flush,
+                               Counted counted)
+    {
+        const uint32_t t = gtid<B>(), lane = t & 31u, w = t >> 5;
+        uint32_t old[MAXEPT];
+        uint4 nd[MAXEPT];
+#pragma unroll
+        for (int r = 0; r < MAXEPT; ++r) {
+            old[r] = kUnvisited;
+            nd[r] = make_uint4(0u, 0u, 0u, 0u);
+            if (c[r] != kUnvisited && PB_CHECK(M.res, c[r] < M.n, 153)) {
+                old[r] = atomicMax(&M.node[c[r]].claim, base);
+                nd[r] = ld_node(M.node + c[r]);
+            }
+        }
+        uint32_t pos[MAXEPT], dsum = 0;
+#pragma unroll
+        for (int r = 0; r < MAXEPT; ++r) {
+            const bool win = old[r] < first;
+            const uint32_t bal = __ballot_sync(kFull, win);
+            pos[r] = __popc(bal & ((1u << lane) - 1u));
+            dsum += win ? nd[r].z : 0u;
+            if (lane == 0)
+                s.wq[r][w] = __popc(bal);
+        }
+        dsum = __reduce_add_sync(kFull, dsum);
+        if (lane == 0)
+            s.tmp32[w] = dsum;
+        gsync<B>();
+        uint32_t Q = 0, Qdeg = 0;
+#pragma unroll
+        for (int i = 0; i < Smem<B, EMAX>::W; ++i)
+            Qdeg += s.tmp32[i];
+#pragma unroll
+        for (int r = 0; r < MAXEPT; ++r) {
+            pos[r] += Q;
+#pragma unroll
+            for (int i = 0; i < Smem<B, EMAX>::W; ++i) {
+                const uint32_t n_ = s.wq[r][i];
+                pos[r] += (uint32_t)i < w ? n_ : 0u;
+                Q += n_;
+            }
+        }
+        if (C.cnt + Q > (uint32_t)EMAX)
+            flush();
+        counted(Agg{C.cnt + Q, C.esum + Qdeg});
+#pragma unroll
+        for (int r = 0; r < MAXEPT; ++r)
+            if (old[r] < first) {
+                const uint32_t at = C.cnt + pos[r];
+                out.node[at] = c[r];
+                out.rs[at] = nd[r].y;
+                out.deg[at] = nd[r].z;
+            }
+        C.cnt += Q;
+        C.esum += Qdeg;
+        gsync<B>();
+    }
+
+    template <typename Flush>
+    __device__ __forceinline__ void collect_any(uint32_t first, const List& out, Agg& C, Flush flush)
+    {
+        uint32_t c[MAXEPT];
+        load_cols(c);
+        claim_list(first, c, out, C, flush, [](const Agg&) {});
+    }
+
+    // Writes the first Q entries of a list to queue positions P0..
+    __device__ void place_list(const List& P, uint32_t P0, uint32_t Q)
+    {
+        for (uint32_t i = gtid<B>(); i < Q; i += B)
+            if (PB_CHECK(M.res, P0 + i < M.n, 154))
+                __stcg(reinterpret_cast<uint4*>(M.rec) + P0 + i, make_uint4(P.node[i], P.rs[i], P.deg[i], 0u));
     }
 
     // The ranked child owning edge offset f: so_eoff[lo] <= f < so_eoff[lo+1].
@@ -1163,7 +1352,7 @@ struct Chunk {
                     const uint32_t c = ld_ro(M.ci + rs + e);
                     if (PB_CHECK(M.res, c < M.n, 122)) {
                         const uint4 nd = ld_node(M.node + c);
-                        if (claim_of(M, nd) == base - 1u - (eb + e)) {
+                        if (nd.x == base - 1u - (eb + e)) {
                             dg[r] = nd.z;
                             ok[r] = true;
                             ++nv;
@@ -1330,8 +1519,7 @@ struct Chunk {
 template <int B, int EMAX, class TeamT>
 __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, unsigned long long* agg,
                          uint32_t& step, const Options& opt, uint32_t start, uint32_t base, bool sorted,
-                         bool write_perm, bool reverse, uint32_t& placed, uint32_t& nlevels, uint32_t& last_start,
-                         uint32_t& wide_f, uint32_t& wide_e)
+                         bool write_perm, bool reverse, uint32_t& placed, uint32_t& nlevels, uint32_t& last_start)
 {
     Chunk<B, EMAX> ch{s, M, base};
     const uint32_t t = gtid<B>();
@@ -1464,8 +1652,6 @@ __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, uns
         }
         // ---- whole team ---------------------------------------------------
         const uint32_t F = st.b - st.a;
-        wide_f = max(wide_f, F);
-        wide_e = max(wide_e, st.Kb - st.Ka);
         const uint32_t p_beg = st.a + (uint32_t)(((uint64_t)F * R) / G);
         const uint32_t p_end = st.a + (uint32_t)(((uint64_t)F * (R + 1)) / G);
         // A1: collect and count.  A CTA whose parents take several chunks
@@ -1510,12 +1696,11 @@ __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, uns
             return false;
         const uint32_t tot_cnt = (uint32_t)(all & 0xFFFFFFFFull);
         const uint32_t tot_esum = (uint32_t)(all >> 32);
-        if (opt.wide_at != 0 && tot_cnt >= opt.wide_at && base == 2u * M.nnz + 3u && M.cf == 0 &&
+        if (opt.wide_at != 0 && tot_cnt >= opt.wide_at && base == 2u * M.nnz + 3u &&
             G == gridDim.x) {
             // a level this wide in the first pass of the whole team (key base
-            // of pass 1 in the main claim word; never a half team, whose
-            // other half would wait for it): the level-synchronous engine
-            // takes the matrix (every CTA has the same totals and leaves)
+            // of pass 1): the level-synchronous engine takes the matrix (every
+            // CTA has the same totals and leaves)
             if (R == 0 && t == 0)
                 set_status(M.res, kNeedWide, 0);
             return false;
@@ -1570,6 +1755,245 @@ __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, uns
     return true;
 }
 
+// One breadth-first pass from `start`, unordered inside a level: what a
+// start-search pass needs while its order does not matter (reorder_matrix).
+// A node's first claim of the pass is the whole dedup.  Levels with a small
+// frontier run on CTA 0 alone, as in bfs_pass, until one is too big; from
+// then on the team works as follows.  A CTA keeps the children it claimed in
+// shared memory and expands them itself in the next level, so a level is one
+// round trip for the claims and one barrier, whose word also carries the
+// level's totals and under which the next columns are loaded (the ordered
+// pass: queue records, columns, node entries, all-gather, claims, barrier).
+// When a CTA's share grows past a chunk it asks, in the same word, for a new
+// split: all lists go to the queue behind an atomic counter and come back in
+// equal runs.  Levels of more than 3/4 of a chunk a CTA go through the queue
+// at once.
+// Grid teams only; no row over EMAX.  first: the smallest key of this pass;
+// base: its largest, the claim of every node.  The last level ends up at
+// queue positions [last_start, placed).
+template <int B, int EMAX>
+__device__ bool level_pass(Smem<B, EMAX>& s, const MatrixView& M, Team& team, const Options& opt, uint32_t start,
+                           uint32_t base, uint32_t first, uint32_t& slot, uint32_t& placed, uint32_t& nlevels,
+                           uint32_t& last_start)
+{
+    Chunk<B, EMAX> ch{s, M, base};
+    using List = typename Chunk<B, EMAX>::List;
+    const uint32_t t = gtid<B>();
+    const uint32_t G = team.size, R = team.rank, n = M.n;
+    const uint4 sn = ld_node(M.node + start);
+    LevelState st;
+    st.a = 0;
+    st.b = 1;
+    st.Ka = 0;
+    st.Kb = sn.z;  // Kb - Ka: entries of the frontier
+    st.L = 0;
+    st.last_start = 0;
+    if (R == 0 && t == 0) {
+        atomicMax(&M.node[start].claim, base);
+        __stcg(reinterpret_cast<uint4*>(M.rec), make_uint4(start, sn.y, sn.z, 0u));
+    }
+    auto is_solo = [&](const LevelState& x) {
+        return G == 1 || ((x.b - x.a) <= opt.solo_parents && (x.Kb - x.Ka) <= opt.solo_edges);
+    };
+    auto next_level = [&](uint32_t cnt, uint32_t esum) {
+        st.last_start = st.b;
+        st.a = st.b;
+        st.b += cnt;
+        st.Ka = st.Kb;
+        st.Kb += esum;
+        st.L += 1;
+    };
+    if (is_solo(st)) {
+        bool ok = true;
+        gsync<B>();
+        if (R == 0) {
+            uint32_t cur = 0, beat = 0;
+            bool listed = false;  // the frontier is in list `cur`
+            while (true) {
+                const List P = ch.list(cur), out = ch.list(cur ^ 1u);
+                uint32_t tail = st.b;  // queue positions taken
+                Agg C{0, 0}, flushed{0, 0};
+                auto flush = [&]() {
+                    ch.place_list(out, tail, C.cnt);
+                    tail += C.cnt;
+                    flushed.esum += C.esum;
+                    C = Agg{0, 0};
+                    gsync<B>();
+                };
+                for (uint32_t p = st.a; p < st.b;) {
+                    p += listed ? ch.form_list(P, p - st.a, st.b - st.a) : ch.form(p, st.b);
+                    ch.collect_any(first, out, C, flush);
+                }
+                const uint32_t cnt = tail - st.b + C.cnt, esum = flushed.esum + C.esum;
+                if (cnt == 0) {
+                    if (listed) {
+                        ch.place_list(P, st.a, st.b - st.a);
+                        gsync<B>();
+                    }
+                    st.a = st.b;  // an empty frontier marks the end of the pass
+                    break;
+                }
+                listed = tail == st.b;
+                cur ^= 1u;
+                next_level(cnt, esum);
+                if (st.b > n) {
+                    set_status(M.res, kErrCheck, 155);
+                    ok = false;
+                    break;
+                }
+                const bool stay = is_solo(st);
+                if (!listed)
+                    flush();
+                else if (!stay)
+                    ch.place_list(out, st.a, cnt);
+                // the others' bounded wait, and an error posted elsewhere:
+                // looked after every few levels
+                if ((++beat & 7u) == 0) {
+                    team.beat();
+                    ok = team.block_ok();
+                }
+                if (!stay || !ok)
+                    break;
+            }
+            gsync<B>();
+            if (G > 1) {
+                if (!team.gate_open(st, ok))
+                    return false;
+            } else if (!ok) {
+                return false;
+            }
+        } else if (!team.gate_wait(st)) {
+            return false;
+        }
+        if (st.a == st.b) {
+            // every CTA leaves the pass together (see bfs_pass)
+            if (G > 1 && !team.sync(8))
+                return false;
+            placed = st.b;
+            nlevels = st.L + 1;
+            last_start = st.last_start;
+            return true;
+        }
+    } else if (!team.sync(2)) {
+        return false;
+    }
+    // ---- the whole team
+    constexpr int MAXEPT = Chunk<B, EMAX>::MAXEPT;
+    uint32_t cur = 0, own = 0;
+    bool listed = false;  // this CTA's share of the level is in list `cur` (own entries, one chunk)
+    uint32_t col[MAXEPT];  // listed: the columns of its edges, on their way
+    while (true) {
+        const uint32_t F = st.b - st.a, E = st.Kb - st.Ka;
+        const List P = ch.list(cur), out = ch.list(cur ^ 1u);
+        Agg C{0, 0};
+        bool split = false;  // some children are in the queue already
+        auto flush = [&]() {
+            if (C.cnt != 0) {
+                if (t == 0)
+                    s.bcast[0] = (uint32_t)atomicAdd(&team.gs->lvl[slot],
+                                                     (unsigned long long)C.esum << 32 | C.cnt);
+                gsync<B>();
+                ch.place_list(out, st.b + s.bcast[0], C.cnt);
+                gsync<B>();
+            }
+            C = Agg{0, 0};
+            split = true;
+        };
+        // the children of this share go through the queue when the level
+        // leaves no room for uneven shares, and a CTA asks for a new split
+        // when its own next share would not fit one chunk (below that a share
+        // costs the same whatever its size)
+        const bool queue = E > G * (uint32_t)(EMAX / 4 * 3);
+        auto too_big = [&](const Agg& g) { return g.cnt > (uint32_t)B || g.esum > (uint32_t)EMAX; };
+        bool arrived = false;
+        if (listed) {
+            if (own != 0) {
+                const bool alone = !queue;
+                ch.claim_list(first, col, out, C, flush, [&](const Agg& g) {
+                    if (alone)
+                        team.level_arrive(g.cnt, g.esum, too_big(g));
+                });
+                arrived = alone;
+            }
+        } else {
+            const uint32_t p_end = st.a + (uint32_t)(((uint64_t)F * (R + 1)) / G);
+            for (uint32_t p = st.a + (uint32_t)(((uint64_t)F * R) / G); p < p_end;) {
+                p += ch.form(p, p_end);
+                ch.collect_any(first, out, C, flush);
+            }
+        }
+        uint32_t cnt = 0, esum = 0;
+        bool keep = false;
+        if (!queue) {
+            const bool ask = split || too_big(C);
+            if (!arrived) {
+                gsync<B>();
+                team.level_arrive(C.cnt, C.esum, ask);
+            }
+            // the next level's columns while the others arrive
+            if (!ask && C.cnt != 0) {
+                ch.form_list(out, 0, C.cnt);
+                ch.load_cols(col);
+            }
+            if (!team.level_wait(5, cnt, esum, keep))
+                return false;
+        }
+        if (keep) {
+            if (cnt == 0) {
+                if (listed) {
+                    // the last level to the queue, for the next start (the
+                    // counter is next used behind another barrier)
+                    if (own != 0) {
+                        if (t == 0)
+                            s.bcast[0] = (uint32_t)atomicAdd(&team.gs->lvl[slot], (unsigned long long)own);
+                        gsync<B>();
+                        ch.place_list(P, st.a + s.bcast[0], own);
+                    }
+                    if (!team.sync(9))
+                        return false;
+                    if (R == 0 && t == 0)
+                        __stcg(&team.gs->lvl[slot], 0ull);
+                }
+                break;
+            }
+            listed = true;
+            own = C.cnt;
+            cur ^= 1u;
+        } else {
+            flush();
+            if (!team.sync(13))
+                return false;
+            const unsigned long long all = __ldcg(&team.gs->lvl[slot]);
+            cnt = (uint32_t)(all & 0xFFFFFFFFull);
+            esum = (uint32_t)(all >> 32);
+            // the counter of the level after next is free (everyone read it
+            // before this barrier): cleared for it
+            slot = slot == 2 ? 0 : slot + 1;
+            if (R == 0 && t == 0)
+                __stcg(&team.gs->lvl[slot == 2 ? 0 : slot + 1], 0ull);
+            if (opt.wide_at != 0 && cnt >= opt.wide_at && base == 2u * M.nnz + 3u && G == gridDim.x) {
+                // a level this wide in the first pass: the level-synchronous
+                // engine takes the matrix (every CTA has the same totals)
+                if (R == 0 && t == 0)
+                    set_status(M.res, kNeedWide, 0);
+                return false;
+            }
+            if (cnt == 0)
+                break;
+            listed = false;
+        }
+        next_level(cnt, esum);
+        if (st.b > n) {
+            set_status(M.res, kErrCheck, 156);
+            return false;
+        }
+    }
+    placed = st.b;
+    nlevels = st.L + 1;
+    last_start = st.last_start;
+    return true;
+}
+
 // Next start of the pseudo-peripheral search (simple_peripheral.cpp:110-127)
 // from the ordered BFS just run: among the last min(outnodes, n-1) positions,
 // those on the last level; the last of minimal valence.  Thread 0 computes.
@@ -1587,6 +2011,24 @@ __device__ __forceinline__ uint32_t next_peripheral_start(const MatrixView& M, u
         }
     }
     return best;
+}
+
+// The node of minimal valence at positions [at, at + width), and how many have
+// that valence (one warp).
+__device__ __forceinline__ uint32_t unique_min_valence(const MatrixView& M, uint32_t at, uint32_t width, uint32_t& node)
+{
+    uint32_t d = kUnvisited, v = 0, same = 0;
+    for (uint32_t i = threadIdx.x & 31u; i < width; i += 32) {
+        const uint4 r = __ldcg(reinterpret_cast<const uint4*>(M.rec) + at + i);
+        same = r.z < d ? 1u : same + (r.z == d ? 1u : 0u);
+        if (r.z < d) {
+            d = r.z;
+            v = r.x;
+        }
+    }
+    const uint32_t dm = __reduce_min_sync(kFull, d);
+    node = __shfl_sync(kFull, v, __ffs(__ballot_sync(kFull, d == dm)) - 1);
+    return __reduce_add_sync(kFull, d == dm ? same : 0u);
 }
 
 // Fills the node table (claim 0, row start, valence) of the matrix.
@@ -1612,7 +2054,7 @@ __device__ void reorder_matrix(Smem<B, EMAX>& s, const MatrixView& M, TeamT& tea
     const uint32_t G = team.size, R = team.rank;
     uint32_t start = opt.start;
     uint32_t passes = 0, ecc = 0, placed = 0, nlevels = 0, last_start = 0;
-    uint32_t step = 0;
+    uint32_t step = 0, slot = 0;
 
     if (start != kUnvisited && start >= n) {
         if (R == 0 && t == 0)
@@ -1624,176 +2066,110 @@ __device__ void reorder_matrix(Smem<B, EMAX>& s, const MatrixView& M, TeamT& tea
     init_nodes<B>(M, R, G);
     if (!team.sync(1))
         return;
-    // pass keys: pass p owns [p*kspan, p*kspan + nnz + 1], separately in
-    // each claim word (claim: start-search and final passes; inv: the
-    // speculative ordered passes)
+    // pass keys: pass p owns [p*kspan, p*kspan + nnz + 1]
     const uint32_t kspan = M.nnz + 2u;
     const uint32_t pmax = (uint32_t)(0xFFFFFFFFull / kspan) - 1u;
-    uint32_t pass_id = 0, pass_id2 = 0;
-
-    // Speculation.  Once the first start-search pass has run, every later
-    // pass may be the last one (its eccentricity equals the previous one);
-    // the final ordered pass then starts from the same node.  So the team
-    // splits in two halves: one runs the start-search pass from the
-    // candidate, the other runs the ordered pass from it at the same time
-    // (claim word inv, queue records rec2, writing the output).  If the
-    // candidate is confirmed, the ordered pass is already done; if not, its
-    // output is overwritten later.  Pays off when most levels are small
-    // enough for one CTA (each half runs them on its first CTA); a level that
-    // needs the whole team takes a half team about 1.5x as long.  Not with
-    // hubs (both halves would share the hub scratch); grid teams only.
-    const bool spec = TeamT::kGrid && M.rec2 != nullptr && G >= 2 && start == kUnvisited && n > 1 &&
-                      opt.mode == kModeFull && __ldcg(&M.res->maxdeg) <= (uint32_t)EMAX;
-    const uint32_t half = G / 2;
-    const bool low = R < half;
-    TeamT sub = team;  // this CTA's half
-    unsigned long long* sub_agg = agg;
-    uint32_t sub_step = 0;
-    if constexpr (TeamT::kGrid) {
-        if (spec) {
-            const size_t pw = team_part_bytes((int)G) / sizeof(unsigned long long);
-            sub_agg = agg + (low ? pw : 2 * pw);
-            sub.size = low ? half : G - half;
-            sub.rank = low ? R : R - half;
-            sub.gs = sub.size > 1 ? team.gs + (low ? 1 : 2) : nullptr;
-            sub.flags = reinterpret_cast<unsigned int*>(sub_agg + 2 * sub.size);
-            sub.expected = sub.size;
-            sub.target = 0;
-            sub.epoch = 0;
-        }
-    }
-    MatrixView M2 = M;  // the speculative ordered pass's view
-    M2.rec = M.rec2;
-    M2.cf = 3;
-    M2.stage = M.stage != nullptr ? M.stage + M.nnz : nullptr;  // its own half of the staging array
-    bool spec_on = false;    // the next search pass runs beside the speculative ordered pass
-    bool solo_dom = false;   // most levels of the first pass ran on one CTA
-    bool narrow = false;     // every team level of the first pass is narrow enough for a half team
-    bool spec_done = false;  // the speculative ordered pass wrote the output
+    uint32_t pass_id = 0;
 
     // pseudo-peripheral search (simple_peripheral.cpp:92-141), then the
-    // degree-sorted pass that writes the permutation.  Every pass goes
-    // through the one call of bfs_pass below (it is large: a single inlined
-    // copy keeps the kernel's registers down).
+    // degree-sorted pass that writes the permutation.
+    //
+    // A search pass has to deliver its level count and the next start, and
+    // that start -- the last node of minimal valence among the last outnodes
+    // discovered, on the last level -- does not depend on the order when the
+    // last level has at most outnodes nodes and one of them alone has the
+    // minimal valence.  So the search runs unordered (level_pass, about half
+    // the time of an ordered level) and only repeats a pass in discovery
+    // order where that fails: never on grids, about a third of the passes of
+    // random geometric graphs.  From the third pass on, which usually
+    // confirms the eccentricity, the search pass is the sorted pass itself
+    // and its order the result if it does.  (Matrices with rows over EMAX and
+    // cluster teams search in discovery order.)
+    enum : uint32_t { kLevels, kFifo, kSorted };
+    const bool any_order = TeamT::kGrid && G <= 255u && __ldcg(&M.res->maxdeg) <= (uint32_t)EMAX;
+    const bool full = opt.mode != kModeStartOnly;
     bool searching = start == kUnvisited && n > 1;
+    bool repeat = false;  // this pass repeats the last one in discovery order
+    uint32_t kind = kSorted, lastdist = 0;
     if (n == 1) {
         // one node: the start search runs one pass and records nothing
         passes = start == kUnvisited ? 1 : 0;
         start = 0;
     } else if (searching) {
         start = n / 2;
+        passes = 1;
+        kind = any_order ? kLevels : kFifo;
     }
-    uint32_t lastdist = 0;
-    while (true) {
-        if (!searching && opt.mode == kModeStartOnly)
-            break;
-        const bool split = searching && spec_on;  // spec_on implies a first pass has run
-        const bool spec_half = split && !low;     // this CTA runs the speculative ordered pass
-        const bool ordered = !searching || spec_half;
-        TeamT& tm = split ? sub : team;
-        unsigned long long* ag = split ? sub_agg : agg;
-        uint32_t& stp = split ? sub_step : step;
-        uint32_t& pid = spec_half ? pass_id2 : pass_id;
-        if (searching)
-            ++passes;
-        if (pid + 1 > pmax) {
-            // reset this pass's claim word (the other half never touches it)
-            const uint32_t cf = spec_half ? 3u : 0u;
-            for (uint64_t v = (uint64_t)tm.rank * B + t; v < n; v += (uint64_t)tm.size * B)
-                reinterpret_cast<uint32_t*>(M.node + v)[cf] = 0u;
-            pid = 0;
-            if (!tm.sync(7))
+    while (searching || full) {
+        if (pass_id + 1 > pmax) {
+            for (uint64_t v = (uint64_t)R * B + t; v < n; v += (uint64_t)G * B)
+                M.node[v].claim = 0u;
+            pass_id = 0;
+            if (!team.sync(7))
                 return;
         }
-        ++pid;
-        const uint32_t base = pid * kspan + M.nnz + 1u;
-        const uint32_t step0 = step;
-        uint32_t pl = 0, nl = 0, ls = 0, wf = 0, we = 0;
-        if (!bfs_pass<B, EMAX>(s, spec_half ? M2 : M, tm, ag, stp, opt, start, base, ordered, ordered,
-                               ordered && opt.reverse != 0, pl, nl, ls, wf, we))
-            return;
-        if (!searching) {
-            placed = pl;
-            nlevels = nl;
-            last_start = ls;
-            break;
-        }
-        uint32_t dist = 0, next = 0;
-        if (!split) {
-            if (pl != n) {
-                if (R == 0 && t == 0)
-                    set_status(M.res, kErrDisconnected, 0);
-                return;
-            }
-            // speculate from the next pass on if at most a quarter of the
-            // levels needed the whole team (step counts them); otherwise from
-            // pass opt.spec_from on, where the search usually ends, if the
-            // widest level takes a CTA of a half team at most four chunks
-            // (measured: the 128^3 grid, 1.6 chunks, gains 14 %; a 1M-node
-            // RGG, 20 chunks, would lose 30 %)
-            if (passes == 1) {
-                solo_dom = 4ull * (step - step0) <= nl;
-                narrow = (uint64_t)wf <= 4ull * half * B && (uint64_t)we <= 4ull * half * EMAX;
-            }
-            spec_on = spec && (solo_dom || (narrow && opt.spec_from != 0 && passes + 1 >= opt.spec_from));
-            dist = nl - 1;
-            if (dist == lastdist) {
-                ecc = dist;
-                searching = false;  // the ordered pass from the same start comes next
-                continue;
-            }
-            if (t == 0)
-                s.bcast[0] = next_peripheral_start(M, opt.outnodes, ls);
-            gsync<B>();
-            next = s.bcast[0];
-            gsync<B>();
-        } else {
+        ++pass_id;
+        const uint32_t base = pass_id * kspan + M.nnz + 1u;
+        // (one call site of each pass: they are large when inlined)
+        if (kind == kLevels) {
             if constexpr (TeamT::kGrid) {
-                // the halves meet in the team's GridSync words st[8..12]
-                if (sub.rank == 0 && t == 0) {
-                    if (low) {
-                        team.gs->st[8] = pl;
-                        team.gs->st[9] = nl;
-                        team.gs->st[10] = pl == n ? next_peripheral_start(M, opt.outnodes, ls) : 0u;
-                    } else {
-                        team.gs->st[11] = pl;
-                        team.gs->st[12] = nl;
-                    }
-                }
-                if (!team.sync(10))
+                if (!level_pass<B, EMAX>(s, M, team, opt, start, base, pass_id * kspan, slot, placed, nlevels,
+                                         last_start))
                     return;
-                const uint32_t pl_u = __ldcg(&team.gs->st[8]), nl_u = __ldcg(&team.gs->st[9]);
-                next = __ldcg(&team.gs->st[10]);
-                const uint32_t pl_s = __ldcg(&team.gs->st[11]), nl_s = __ldcg(&team.gs->st[12]);
-                if (!team.sync(11))  // everyone has read st[8..12] before the next round writes them
-                    return;
-                if (pl_u != n) {
-                    if (R == 0 && t == 0)
-                        set_status(M.res, kErrDisconnected, 0);
-                    return;
-                }
-                if (pl_s != n || nl_s != nl_u) {  // same start, same levels: cannot differ
-                    if (R == 0 && t == 0)
-                        set_status(M.res, kErrCheck, 4);
-                    return;
-                }
-                dist = nl_u - 1;
-                if (dist == lastdist) {
-                    ecc = dist;
-                    placed = pl_s;
-                    nlevels = nl_s;
-                    spec_done = true;
-                    break;
-                }
+            }
+        } else if (!bfs_pass<B, EMAX>(s, M, team, agg, step, opt, start, base, kind == kSorted, kind == kSorted,
+                                      kind == kSorted && opt.reverse != 0, placed, nlevels, last_start)) {
+            return;
+        }
+        if (!searching)
+            break;
+        if (placed != n) {
+            if (R == 0 && t == 0)
+                set_status(M.res, kErrDisconnected, 0);
+            return;
+        }
+        const uint32_t dist = nlevels - 1;
+        if (dist == lastdist && !repeat) {
+            ecc = dist;
+            searching = false;
+            if (kind == kSorted)
+                break;  // confirmed by the sorted pass: the result
+            kind = kSorted;  // the sorted pass from the same start comes next
+            continue;
+        }
+        // the next start (every CTA finds the same)
+        const uint32_t width = n - last_start;
+        if (kind == kFifo) {
+            if (t == 0) {
+                s.bcast[0] = next_peripheral_start(M, opt.outnodes, last_start);
+                s.bcast[1] = 1u;
+            }
+        } else if (t < 32) {
+            uint32_t v = 0, count = 0;
+            if (width <= min(opt.outnodes, n - 1))
+                count = unique_min_valence(M, last_start, width, v);
+            if (t == 0) {
+                s.bcast[0] = v;
+                s.bcast[1] = count == 1u ? 1u : 0u;
             }
         }
+        gsync<B>();
+        const uint32_t next = s.bcast[0];
+        repeat = s.bcast[1] == 0u;
+        gsync<B>();
+        if (repeat) {
+            kind = kFifo;
+            continue;
+        }
+        start = next;
+        lastdist = dist;
         if (passes > n) {  // eccentricities only grow; cannot happen on a valid run
             if (R == 0 && t == 0)
                 set_status(M.res, kErrCheck, 3);
             return;
         }
-        start = next;
-        lastdist = dist;
+        ++passes;
+        kind = passes >= 3 && full ? kSorted : any_order ? kLevels : kFifo;
     }
     if (opt.mode == kModeStartOnly) {
         if (R == 0 && t == 0) {
@@ -1811,12 +2187,10 @@ __device__ void reorder_matrix(Smem<B, EMAX>& s, const MatrixView& M, TeamT& tea
         }
         return;
     }
-    const PosRec* final_rec = spec_done ? M.rec2 : M.rec;
-
     if (opt.want_bw) {
         // inverse permutation (CM positions) into node[].inv
         for (uint64_t pos = (uint64_t)R * B + t; pos < n; pos += (uint64_t)G * B) {
-            const uint4 r = __ldcg(reinterpret_cast<const uint4*>(final_rec) + pos);
+            const uint4 r = __ldcg(reinterpret_cast<const uint4*>(M.rec) + pos);
             M.node[r.x].inv = (uint32_t)pos;
         }
         if (!team.sync(6))

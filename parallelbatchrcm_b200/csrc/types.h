@@ -46,13 +46,17 @@ struct alignas(16) NodeEntry {
 //   heartbeat  bumped by CTA 0 once per solo level (keeps the waiters' bounded
 //              wait from running out while CTA 0 makes progress)
 //   st[]       the level state CTA 0 publishes with the epoch
+//   lvl[]      counters the CTAs append their children behind (level_pass)
+//   word[]     its barrier words
 struct alignas(128) GridSync {
     unsigned int count;
     unsigned int pad0[31];
     unsigned int epoch;
     unsigned int heartbeat;
     unsigned int st[14];
-    unsigned int pad1[16];
+    unsigned long long lvl[3];  // unordered passes: (edges << 32 | nodes) of the level being filled, in rotation
+    unsigned long long word[3];  // unordered passes: barrier words (Team::level_sync)
+    unsigned int pad1[4];
 };
 
 // Device-side result of one matrix.
@@ -86,10 +90,7 @@ struct MatrixView {
     uint32_t* perm;                    // n   output
     uint32_t* hub;                     // 4 * nnz hub scratch, or nullptr if no hub can occur
     DevResult* res;
-    PosRec* rec2;                      // n: queue records of the speculative ordered pass, or nullptr
-    uint32_t cf;                       // claim word of NodeEntry this pass uses (0 claim, 3 inv)
-    PosRec* stage;                     // 2 nnz: ranked children of multi-chunk team levels (the
-                                       // speculative half uses the second nnz), or nullptr
+    PosRec* stage;                     // nnz: ranked children of multi-chunk team levels, or nullptr
 };
 
 constexpr uint64_t kMaxNnz = 0xFFFFFFF0ull;
@@ -107,16 +108,6 @@ constexpr uint32_t kSoloMaxNodes = 1u << 20;
 inline size_t team_words_bytes(int ctas)
 {
     return 16 * (size_t)(ctas > 0 ? ctas : 1) + 4 * ((size_t)(ctas > 0 ? ctas : 1) + 8);
-}
-
-// A single-matrix team launch gets kTeamParts sets of team words and
-// GridSyncs: part 0 for the whole team, parts 1 and 2 for its two halves
-// while they run a start-search pass and the speculative ordered pass side
-// by side.  Parts are team_part_bytes apart.
-constexpr int kTeamParts = 3;
-PBRCM_HD inline size_t team_part_bytes(int ctas)
-{
-    return (16 * (size_t)(ctas > 0 ? ctas : 1) + 4 * ((size_t)(ctas > 0 ? ctas : 1) + 8) + 255) & ~(size_t)255;
 }
 
 // One matrix of a batch: its view, its team size (CTAs that reorder it
@@ -150,7 +141,6 @@ struct Options {
     uint32_t solo_edges;    // a level with at most this many edges runs on CTA 0 alone
     uint32_t solo_parents;  // ... and at most this many parents
     uint32_t barrier;       // team barrier: 0 counter, 1 flag array
-    uint32_t spec_from;     // speculative split from this search pass on (0: only for solo-dominated matrices)
     uint32_t wide_at;       // first BFS pass (key base 2 nnz + 3): a level of at least this many nodes
                             // hands the matrix to the level-synchronous engine (kNeedWide; 0 = never)
     unsigned long long data_wait_ns;  // batch kernels: bound of the wait for a matrix's CSR to arrive
