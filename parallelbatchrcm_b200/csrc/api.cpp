@@ -451,23 +451,25 @@ int32_t Context::run_single(const uint32_t* rp, const uint32_t* ci, uint32_t n, 
     return PBRCM_OK;
 }
 
-// inv (n) | scan partials | mid-row list (n) | long-row list | counters
+// inv (n) | row starts (n) | scan partials | mid-row list (n) | long-row list | counters
 size_t Context::permute_work_bytes(uint32_t n, uint64_t nnz)
 {
-    return 2 * al256(4 * (size_t)n) + al256(4 * (size_t)scan_partials_count(n)) +
+    return 3 * al256(4 * (size_t)n) + al256(4 * (size_t)scan_partials_count(n)) +
            al256(4 * (size_t)permute_long_cap(n, nnz)) + 256;
 }
 
-// B = P A P^T into out_*, after the CSR check on the same stream (the
-// permutation kernels bound every access themselves, so they need not wait
-// for its verdict); one synchronisation of `st`, two if a row has more than
-// 1,024 entries and the long-row scratch has to be allocated first.
+// B = P A P^T into out_*; the permutation kernels check the CSR and the
+// permutation as they read them (and bound every access themselves, so none
+// waits for a verdict); one synchronisation of `st`, two if a row has more
+// than 1,024 entries and the long-row scratch has to be allocated first.
 int32_t Context::run_permute(const uint32_t* rp, const uint32_t* ci, const void* vals, uint32_t val_bytes, uint32_t n,
                              uint64_t nnz, const uint32_t* perm, uint32_t* out_rp, uint32_t* out_ci, void* out_vals,
                              uint32_t* out_map, unsigned char* work, cudaStream_t st)
 {
     size_t o = 0;
     uint32_t* inv = reinterpret_cast<uint32_t*>(work + o);
+    o += al256(4 * (size_t)n);
+    uint32_t* beg = reinterpret_cast<uint32_t*>(work + o);
     o += al256(4 * (size_t)n);
     uint32_t* partials = reinterpret_cast<uint32_t*>(work + o);
     o += al256(4 * (size_t)scan_partials_count(n));
@@ -479,8 +481,7 @@ int32_t Context::run_permute(const uint32_t* rp, const uint32_t* ci, const void*
     const uint32_t cap_long = permute_long_cap(n, nnz);
     uint32_t* scratch = d_hub != nullptr && cap_hub >= 4 * (size_t)std::max<uint64_t>(nnz, 1) ? d_hub : nullptr;
     if (cudaMemsetAsync(d_res, 0, sizeof(DevResult), st) != cudaSuccess ||
-        launch_validate(rp, ci, n, (uint32_t)nnz, d_res, sms, st) != cudaSuccess ||
-        launch_permute(rp, ci, vals, val_bytes, n, (uint32_t)nnz, perm, inv, out_rp, out_ci, out_vals, out_map,
+        launch_permute(rp, ci, vals, val_bytes, n, (uint32_t)nnz, perm, inv, beg, out_rp, out_ci, out_vals, out_map,
                        partials, mids, longs, cap_long, counters, scratch, d_res, sms, st) != cudaSuccess ||
         cudaMemcpyAsync(h_res, d_res, sizeof(DevResult), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaMemcpyAsync(h_aux, counters, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

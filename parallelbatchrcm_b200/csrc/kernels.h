@@ -88,19 +88,16 @@ int cluster_max_active(int p, int csize);  // co-resident clusters of that size
 cudaError_t launch_cluster(int p, const BatchJob* jobs, uint32_t nbig, const BatchSlot* slots, uint32_t nslots,
                            uint32_t* counters, const Options& copt, const Options& opt, int csize, int nclusters,
                            cudaStream_t st);
-// inv[perm[k]] = k over a zeroed-to-0xFF inv; a non-permutation posts
-// kErrArg (kernels.cu)
-void launch_perm_inverse(const uint32_t* perm, uint32_t n, uint32_t* inv, DevResult* res, int blocks,
-                         cudaStream_t st);
 // B = P A P^T (permute.cu): row_ptr_out (n+1), col_idx_out (nnz), values of
 // val_bytes 0 / 4 / 8 and the source map (nullable) from row_ptr, col_idx,
-// values and perm.  Workspace: inv (n), partials (scan_partials_count(n)),
+// values and perm, which it checks (kErrArg).  Workspace: inv (n), beg (n),
+// partials (scan_partials_count(n)),
 // mid_rows (n), long_rows (cap_long = permute_long_cap(n, nnz)), counters
 // (2), scratch (4 * nnz, only needed when a row has more than 1,024
 // entries; else nullptr and cap_long 0).
 cudaError_t launch_permute(const uint32_t* rp, const uint32_t* ci, const void* vals, uint32_t val_bytes, uint32_t n,
-                           uint32_t nnz, const uint32_t* perm, uint32_t* inv, uint32_t* out_rp, uint32_t* out_ci,
-                           void* out_vals, uint32_t* out_map, uint32_t* partials, uint32_t* mid_rows,
+                           uint32_t nnz, const uint32_t* perm, uint32_t* inv, uint32_t* beg, uint32_t* out_rp,
+                           uint32_t* out_ci, void* out_vals, uint32_t* out_map, uint32_t* partials, uint32_t* mid_rows,
                            uint32_t* long_rows, uint32_t cap_long, uint32_t* counters, uint32_t* scratch,
                            DevResult* res, int sms, cudaStream_t st);
 // the long rows launch_permute listed (counters[1]) when it had no scratch
@@ -117,7 +114,8 @@ cudaError_t launch_scan(uint32_t* data, uint64_t m, uint32_t* partials, cudaStre
 // (writes at or past cap dropped) from a symmetric CSR with sorted rows.
 // Workspace: parent (n), partials (scan_partials_count(n)), counters (4):
 // [0] first non-empty row, [1] links added, [2] check flags (1 column out of
-// range, 2 row not sorted, 4 not symmetric, 8 union limit).
+// range or bad row pointers, 2 row not sorted, 4 not symmetric, 8 union limit),
+// [3] distinct entries below the diagonal less those above it (not 0: not symmetric).
 cudaError_t launch_connect(const uint32_t* rp, const uint32_t* ci, uint32_t n, uint32_t nnz, uint32_t* out_rp,
                            uint32_t* out_ci, uint64_t cap, uint32_t* parent, uint32_t* partials, uint32_t* counters,
                            int sms, cudaStream_t st);
