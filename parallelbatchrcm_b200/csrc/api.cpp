@@ -507,9 +507,8 @@ size_t Context::connect_work_bytes(uint32_t n)
     return al256(4 * (size_t)n) + al256(4 * (size_t)scan_partials_count(n)) + 256;
 }
 
-// The loader's connectivity repair into out_* after the CSR check on the same
-// stream (the repair kernels clamp every row range themselves); one
-// synchronisation of `st`.
+// The loader's connectivity repair into out_*; its kernels check the CSR as
+// they read it and clamp every row range; one synchronisation of `st`.
 int32_t Context::run_connect(const uint32_t* rp, const uint32_t* ci, uint32_t n, uint64_t nnz, uint32_t* out_rp,
                              uint32_t* out_ci, uint64_t cap, uint64_t* nnz_out, uint32_t* links_out,
                              unsigned char* work, cudaStream_t st)
@@ -518,18 +517,13 @@ int32_t Context::run_connect(const uint32_t* rp, const uint32_t* ci, uint32_t n,
     uint32_t* partials = reinterpret_cast<uint32_t*>(work + al256(4 * (size_t)n));
     uint32_t* counters =
         reinterpret_cast<uint32_t*>(work + al256(4 * (size_t)n) + al256(4 * (size_t)scan_partials_count(n)));
-    if (cudaMemsetAsync(d_res, 0, sizeof(DevResult), st) != cudaSuccess ||
-        launch_validate(rp, ci, n, (uint32_t)nnz, d_res, sms, st) != cudaSuccess ||
-        launch_connect(rp, ci, n, (uint32_t)nnz, out_rp, out_ci, cap, parent, partials, counters, sms, st) !=
+    if (launch_connect(rp, ci, n, (uint32_t)nnz, out_rp, out_ci, cap, parent, partials, counters, sms, st) !=
             cudaSuccess ||
-        cudaMemcpyAsync(h_res, d_res, sizeof(DevResult), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaMemcpyAsync(h_aux, counters, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaMemcpyAsync(h_aux, counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
         return PBRCM_ERR_CUDA;
-    if (h_res->status != kOk)
-        return map_status(h_res->status);
-    if (h_aux[2] != 0)
-        return PBRCM_ERR_ARG;  // column out of range, unsorted row or not symmetric
+    if (h_aux[2] != 0 || h_aux[3] != 0)
+        return PBRCM_ERR_ARG;  // bad row pointers or columns, unsorted row or not symmetric
     if (h_aux[0] >= n)
         return PBRCM_ERR_FORMAT;  // no entry at all
     const uint64_t need = nnz + 2ull * h_aux[1];

@@ -13,18 +13,26 @@
 // an empty row, which it queues without marking; the host loader of this
 // library and this pass link it like any other component.)
 //
-// Passes (all HBM-bound, one thread per 8 consecutive entries or per row):
+// Passes (a warp takes 32 rows at a time and deals their entries out to its
+// lanes, so that no entry searches row_ptr for its row; in the hook pass a
+// lane has four entries' chains of dependent loads in flight):
 //   1. k_cc_init: parent[v] = min(v, first column of row v) (rows are sorted,
-//      so that is the smallest neighbour) and minn;
+//      so that is the smallest neighbour) and minn; checks the row pointers;
+//      k_cc_flatten: every node under its root in that forest;
 //   2. k_cc_hook: union-find over the entries (u, v), u < v, hooking the
 //      larger root under the smaller with atomicCAS and halving paths on the
 //      way up -- the minimum-label form of the ECL-CC algorithm (Jaiganesh and
 //      Burtscher, HPDC 2018), so that each component's root is its smallest
 //      node and "m is a component minimum" is parent[m] == m afterwards.  The
 //      same pass checks each entry: column in range, row sorted, and the
-//      transposed entry present (the repair is defined on symmetric patterns);
+//      pattern symmetric (the repair is defined on symmetric patterns): every
+//      entry left of the diagonal has its transposed entry, and there are as
+//      many distinct entries right of it, so those have theirs too -- half the
+//      random searches of checking every entry.  The unions that are left are dealt
+//      out to the lanes (each a chain of dependent loads; one after the other they
+//      took 375 us of 15M entries, side by side 284);
 //   3. k_connect_rowlen: row length plus the links of the row (at most two),
-//      scanned into row_ptr_out (the three scan kernels of permute.cu);
+//      scanned into row_ptr_out (the scan kernels of permute.cu);
 //   4. k_connect_copy: each entry shifted to its place in the output row, then
 //      each link inserted at its sorted position.
 #include <algorithm>
@@ -39,14 +47,15 @@ namespace pbrcm {
 
 namespace {
 
-constexpr int kEntriesPerThread = 8;
 constexpr int kThreads = 256;
+constexpr int kInFlight = 4;  // entries a lane of the hook pass works on at once
 
-// counters[0] minn, [1] links, [2] check flags
+// counters[0] minn, [1] links, [2] check flags, [3] distinct entries left of
+// the diagonal less those right of it
 constexpr uint32_t kFlagRange = 1, kFlagUnsorted = 2, kFlagAsym = 4, kFlagDepth = 8;
 
-// Row v's entry range, clamped into [0, nnz] (the CSR check runs beside these
-// kernels on the same stream; a bad row_ptr must not send them out of bounds).
+// Row v's entry range, clamped into [0, nnz] (a bad row_ptr must not send a
+// kernel out of bounds before the call's verdict is read).
 __device__ __forceinline__ void row_range(const uint32_t* __restrict__ rp, uint32_t v, uint32_t nnz, uint32_t& b,
                                           uint32_t& e)
 {
@@ -54,19 +63,31 @@ __device__ __forceinline__ void row_range(const uint32_t* __restrict__ rp, uint3
     e = min(max(rp[v + 1], b), nnz);
 }
 
-// The row containing entry k: the largest v < n with rp[v] <= k.
-__device__ __forceinline__ uint32_t row_of(const uint32_t* __restrict__ rp, uint32_t n, uint32_t k)
-{
-    uint32_t lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const uint32_t mid = lo + (hi - lo + 1) / 2;
-        if (rp[mid] <= k)
-            lo = mid;
-        else
-            hi = mid - 1;
+// The 32 rows from v0 on, one per lane (empty past n).
+struct RowTile {
+    uint32_t b, e;      // this lane's row
+    uint32_t beg, end;  // entries of the tile
+    __device__ __forceinline__ RowTile(const uint32_t* __restrict__ rp, uint32_t n, uint32_t nnz, uint32_t v0)
+    {
+        const uint32_t lane = threadIdx.x & 31u;
+        const uint64_t v = (uint64_t)v0 + lane;
+        b = e = min(rp[n], nnz);
+        if (v < n)
+            row_range(rp, (uint32_t)v, nnz, b, e);
+        beg = __shfl_sync(kFull, b, 0);
+        end = __shfl_sync(kFull, e, 31);
     }
-    return lo;
-}
+    // The lane whose row holds entry k: the last with b <= k (by the whole
+    // warp; k past the end names some lane).
+    __device__ __forceinline__ uint32_t lane_of(uint32_t k) const
+    {
+        uint32_t l = 0;
+#pragma unroll
+        for (uint32_t d = 16; d > 0; d >>= 1)
+            l = __shfl_sync(kFull, b, l + d) <= k ? l + d : l;
+        return l;
+    }
+};
 
 // First index in ci[b, e) whose column is >= x (a sorted row).
 __device__ __forceinline__ uint32_t lower_bound(const uint32_t* __restrict__ ci, uint32_t b, uint32_t e, uint32_t x)
@@ -159,10 +180,13 @@ __global__ void __launch_bounds__(kThreads) k_cc_init(const uint32_t* __restrict
                                                       uint32_t* counters)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    uint32_t first = kFull;
+    uint32_t first = kFull, flags = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const uint32_t v = (uint32_t)i;
         uint32_t b, e;
+        const uint32_t b0 = rp[v], e0 = rp[v + 1];
+        if (e0 < b0 || e0 > nnz || (v == 0 && b0 != 0) || (v == n - 1 && e0 != nnz))
+            flags |= kFlagRange;
         row_range(rp, v, nnz, b, e);
         uint32_t p = v;
         if (e > b) {
@@ -176,52 +200,133 @@ __global__ void __launch_bounds__(kThreads) k_cc_init(const uint32_t* __restrict
     first = __reduce_min_sync(0xFFFFFFFFu, first);
     if ((threadIdx.x & 31) == 0 && first != kFull)
         atomicMin(counters, first);
+    flags = __reduce_or_sync(0xFFFFFFFFu, flags);
+    if ((threadIdx.x & 31) == 0 && flags)
+        atomicOr(counters + 2, flags);
+}
+
+// parent[v] = root of v in the forest of first columns (k_cc_init), so that
+// most entries of the hook pass find both ends under one root and the others
+// start their climb at one.
+__global__ void __launch_bounds__(kThreads) k_cc_flatten(uint32_t n, uint32_t* parent)
+{
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
+        uint32_t p = __ldcg(parent + v);
+        for (uint32_t g = __ldcg(parent + p); g != p; g = __ldcg(parent + p))
+            p = g;
+        parent[v] = p;
+    }
 }
 
 __global__ void __launch_bounds__(kThreads) k_cc_hook(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
                                                       uint32_t n, uint32_t nnz, uint32_t* parent, uint32_t* counters)
 {
-    const uint64_t chunks = ((uint64_t)nnz + kEntriesPerThread - 1) / kEntriesPerThread;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    uint32_t flags = 0;
-    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < chunks; t += stride) {
-        const uint32_t k0 = (uint32_t)(t * kEntriesPerThread);
-        const uint32_t k1 = (uint32_t)min((uint64_t)k0 + kEntriesPerThread, (uint64_t)nnz);
-        uint32_t v = row_of(rp, n, k0);
-        uint32_t b, e;
-        row_range(rp, v, nnz, b, e);
-        uint32_t prev = k0 > b && k0 - 1 < e ? ci[k0 - 1] : 0u;
-        for (uint32_t k = k0; k < k1; ++k) {
-            while (k >= e && v + 1 < n) {  // next non-empty row
-                ++v;
-                row_range(rp, v, nnz, b, e);
+    constexpr int U = kInFlight;
+    if (__ldcg(counters + 2) & kFlagRange)
+        return;  // bad row pointers (k_cc_init): the tiles need not partition the entries
+    const uint32_t lane = threadIdx.x & 31u;
+    __shared__ uint2 pair_list[kThreads / 32][32 * U];
+    uint2* const list = pair_list[threadIdx.x >> 5];
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    uint32_t flags = 0, lower = 0;
+    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32 < n; w += nwarps) {
+        const uint32_t v0 = (uint32_t)(w * 32);
+        const RowTile t(rp, n, nnz, v0);
+        for (uint32_t k0 = t.beg; k0 < t.end; k0 += 32u * U) {
+            uint32_t v[U], u[U], ub[U], ue[U];
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+                const uint32_t k = k0 + 32u * i + lane;
+                const uint32_t l = t.lane_of(k);
+                const uint32_t b = __shfl_sync(kFull, t.b, l), e = __shfl_sync(kFull, t.e, l);
+                v[i] = v0 + l;
+                u[i] = v[i];  // nothing to do
+                if (k < t.end) {
+                    if (k < b || k >= e) {  // only a bad row_ptr leaves k outside every row
+                        flags |= kFlagRange;
+                    } else {
+                        const uint32_t c = ci[k], prev = k > b ? ci[k - 1] : kFull;
+                        if (c >= n)
+                            flags |= kFlagRange;
+                        else if (c < v[i])
+                            u[i] = c;
+                        if (k > b && prev > c)
+                            flags |= kFlagUnsorted;
+                        if (prev != c)
+                            lower += c < v[i] ? 1u : c > v[i] ? 0xFFFFFFFFu : 0u;
+                    }
+                }
             }
-            if (k < b || k >= e) {  // only a bad row_ptr leaves k outside every row
-                flags |= kFlagRange;
-                break;
+            // the neighbours' rows, and both ends' parents
+            uint32_t pu[U], pv[U];
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+                ub[i] = ue[i] = pu[i] = pv[i] = 0;
+                if (u[i] != v[i]) {
+                    row_range(rp, u[i], nnz, ub[i], ue[i]);
+                    pu[i] = __ldcg(parent + u[i]);
+                    pv[i] = __ldcg(parent + v[i]);
+                }
             }
-            const uint32_t u = ci[k];
-            if (u >= n) {
-                flags |= kFlagRange;
-                continue;
+            // the transposed entry: four columns of each neighbour's row at a
+            // time (rows are short), a longer row narrowed first
+#pragma unroll
+            for (int i = 0; i < U; ++i)
+                while (ue[i] - ub[i] > 16) {
+                    const uint32_t mid = ub[i] + (ue[i] - ub[i]) / 2;
+                    if (ci[mid] <= v[i])
+                        ub[i] = mid;
+                    else
+                        ue[i] = mid;
+                }
+            bool more = true;
+            while (__any_sync(kFull, more)) {
+                uint32_t x[U][4];
+#pragma unroll
+                for (int i = 0; i < U; ++i)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        x[i][q] = ub[i] + q < ue[i] ? ci[ub[i] + q] : kFull;
+                more = false;
+#pragma unroll
+                for (int i = 0; i < U; ++i) {
+                    // found: an empty range, with the row's end as a mark
+                    if (x[i][0] == v[i] || x[i][1] == v[i] || x[i][2] == v[i] || x[i][3] == v[i])
+                        ub[i] = ue[i] = kFull;
+                    else if (ub[i] < ue[i])
+                        ub[i] = min(ub[i] + 4, ue[i]);
+                    more |= ub[i] < ue[i];
+                }
             }
-            if (k > b && prev > u)
-                flags |= kFlagUnsorted;
-            prev = u;
-            if (u == v)
-                continue;
-            uint32_t ub, ue;
-            row_range(rp, u, nnz, ub, ue);
-            const uint32_t at = lower_bound(ci, ub, ue, v);
-            if (at >= ue || ci[at] != v)
-                flags |= kFlagAsym;
-            if (u < v && !cc_unite(parent, u, v, n))
-                flags |= kFlagDepth;
+            // the pairs to join (two ends under one parent are one component
+            // already), side by side
+            uint32_t pairs = 0;
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+                if (u[i] != v[i] && ub[i] != kFull)
+                    flags |= kFlagAsym;
+                const bool need = u[i] != v[i] && pu[i] != pv[i];
+                const uint32_t bal = __ballot_sync(kFull, need);
+                if (need)
+                    list[pairs + __popc(bal & ((1u << lane) - 1u))] = make_uint2(pu[i], pv[i]);
+                pairs += __popc(bal);
+            }
+            __syncwarp();
+            for (uint32_t i = lane; i < pairs; i += 32) {
+                const uint2 p = list[i];
+                if (!cc_unite(parent, p.x, p.y, n))
+                    flags |= kFlagDepth;
+            }
+            __syncwarp();
         }
     }
     flags = __reduce_or_sync(0xFFFFFFFFu, flags);
-    if ((threadIdx.x & 31) == 0 && flags)
+    lower = __reduce_add_sync(0xFFFFFFFFu, lower);
+    if (lane == 0 && flags)
         atomicOr(counters + 2, flags);
+    if (lane == 0 && lower)
+        atomicAdd(counters + 3, lower);
 }
 
 // out_rp[v + 1] = length of row v + its links; counters[1] = number of links.
@@ -256,43 +361,47 @@ __global__ void __launch_bounds__(kThreads) k_connect_copy(const uint32_t* __res
                                                            const uint32_t* counters, const uint32_t* __restrict__ out_rp,
                                                            uint32_t* __restrict__ out_ci, uint64_t cap)
 {
+    constexpr int U = 4;
+    if (__ldcg(counters + 2) != 0)
+        return;  // the call fails
     const uint32_t minn = __ldcg(counters);
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t chunks = ((uint64_t)nnz + kEntriesPerThread - 1) / kEntriesPerThread;
-    for (uint64_t t = tid; t < chunks; t += stride) {
-        const uint32_t k0 = (uint32_t)(t * kEntriesPerThread);
-        const uint32_t k1 = (uint32_t)min((uint64_t)k0 + kEntriesPerThread, (uint64_t)nnz);
-        uint32_t v = row_of(rp, n, k0);
-        uint32_t b, e, lk[2];
-        row_range(rp, v, nnz, b, e);
-        int nl = out_rp[v + 1] - out_rp[v] != e - b ? row_links(parent, n, minn, v, lk) : 0;
-        uint64_t base = (uint64_t)out_rp[v] - b;
-        for (uint32_t k = k0; k < k1; ++k) {
-            while (k >= e && v + 1 < n) {
-                ++v;
-                row_range(rp, v, nnz, b, e);
-                nl = out_rp[v + 1] - out_rp[v] != e - b ? row_links(parent, n, minn, v, lk) : 0;
-                base = (uint64_t)out_rp[v] - b;
-            }
-            if (k < b || k >= e)
-                break;
-            const uint32_t c = ci[k];
-            const uint64_t at = base + k + (nl > 0 && lk[0] < c ? 1 : 0) + (nl > 1 && lk[1] < c ? 1 : 0);
-            if (at < cap)
-                out_ci[at] = c;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32 < n; w += nwarps) {
+        const uint32_t v0 = (uint32_t)(w * 32);
+        const RowTile t(rp, n, nnz, v0);
+        uint32_t ob = 0, lk[2] = {0, 0};
+        int nl = 0;
+        if (v0 + (uint64_t)lane < n) {
+            ob = out_rp[v0 + lane];
+            if (out_rp[v0 + lane + 1] - ob != t.e - t.b)
+                nl = row_links(parent, n, minn, v0 + lane, lk);
         }
-    }
-    for (uint64_t i = tid; i < n; i += stride) {
-        const uint32_t v = (uint32_t)i;
-        uint32_t lk[2];
-        const int nl = row_links(parent, n, minn, v, lk);
-        if (nl == 0)
-            continue;
-        uint32_t b, e;
-        row_range(rp, v, nnz, b, e);
+        const bool links = __any_sync(kFull, nl != 0);
+        for (uint32_t k0 = t.beg; k0 < t.end; k0 += 32u * U) {
+            uint32_t c[U], l[U];
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+                const uint32_t k = k0 + 32u * i + lane;
+                l[i] = t.lane_of(k);
+                c[i] = k < t.end ? ci[k] : 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+                const uint32_t k = k0 + 32u * i + lane;
+                const uint32_t b = __shfl_sync(kFull, t.b, l[i]), e = __shfl_sync(kFull, t.e, l[i]);
+                uint64_t at = (uint64_t)__shfl_sync(kFull, ob, l[i]) + (k - b);
+                if (links) {
+                    const int ln = __shfl_sync(kFull, nl, l[i]);
+                    const uint32_t l0 = __shfl_sync(kFull, lk[0], l[i]), l1 = __shfl_sync(kFull, lk[1], l[i]);
+                    at += (ln > 0 && l0 < c[i] ? 1 : 0) + (ln > 1 && l1 < c[i] ? 1 : 0);
+                }
+                if (k < t.end && k >= b && k < e && at < cap)
+                    out_ci[at] = c[i];
+            }
+        }
         for (int j = 0; j < nl; ++j) {
-            const uint64_t at = (uint64_t)out_rp[v] + (lower_bound(ci, b, e, lk[j]) - b) + j;
+            const uint64_t at = (uint64_t)ob + (lower_bound(ci, t.b, t.e, lk[j]) - t.b) + j;
             if (at < cap)
                 out_ci[at] = lk[j];
         }
@@ -307,22 +416,23 @@ cudaError_t launch_connect(const uint32_t* rp, const uint32_t* ci, uint32_t n, u
 {
     const int rows_blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n + kThreads - 1) / kThreads,
                                                                           (uint64_t)sms * 8));
-    const uint64_t chunks = ((uint64_t)nnz + kEntriesPerThread - 1) / kEntriesPerThread;
-    const int entry_blocks =
-        (int)std::max<uint64_t>(1, std::min<uint64_t>((chunks + kThreads - 1) / kThreads, (uint64_t)sms * 16));
+    // the passes over entries: a warp per 32 rows
+    const int tile_blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n + kThreads - 1) / kThreads,
+                                                                          (uint64_t)sms * 16));
     cudaError_t e = cudaMemsetAsync(counters, 0xFF, sizeof(uint32_t), st);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(counters + 1, 0, 3 * sizeof(uint32_t), st);
     if (e != cudaSuccess)
         return e;
     k_cc_init<<<rows_blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters);
+    k_cc_flatten<<<rows_blocks, kThreads, 0, st>>>(n, parent);
     if (nnz > 0)
-        k_cc_hook<<<entry_blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters);
+        k_cc_hook<<<tile_blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters);
     k_connect_rowlen<<<rows_blocks, kThreads, 0, st>>>(rp, n, nnz, parent, counters, out_rp);
     e = launch_scan(out_rp + 1, n, partials, st);
     if (e != cudaSuccess)
         return e;
-    k_connect_copy<<<std::max(entry_blocks, rows_blocks), kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters,
+    k_connect_copy<<<tile_blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters,
                                                                              out_rp, out_ci, cap);
     return cudaGetLastError();
 }

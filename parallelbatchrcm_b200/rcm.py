@@ -498,14 +498,15 @@ def connect_device(row_ptr_t, col_idx_t, *, cap: int | None = None, ctx: Context
     include/Graph.h:160-263) on device-resident torch tensors of a symmetric
     pattern with sorted rows.  Returns (row_ptr, col_idx, links): the joined
     CSR on the same device and the number of links added.  The output is
-    first given room for `cap` entries (default: nnz plus a small slack) and
-    reallocated to the exact size if the matrix needs more."""
+    first given room for `cap` entries (default: nnz plus two for every fourth
+    node, so that the repair runs once unless components are smaller than
+    that) and reallocated to the exact size if the matrix needs more."""
     import torch
 
     n, nnz = row_ptr_t.numel() - 1, col_idx_t.numel()
     dev = row_ptr_t.device
     orp = torch.empty(n + 1, dtype=torch.int32, device=dev)
-    room = cap if cap is not None else nnz + 2 * min(max(n - 1, 0), max(1024, n // 64))
+    room = cap if cap is not None else nnz + 2 * min(max(n - 1, 0), max(1024, n // 4))
     st = stream.cuda_stream if stream is not None else torch.cuda.current_stream(dev).cuda_stream
     L = _lib.lib()
     for _ in range(2):
