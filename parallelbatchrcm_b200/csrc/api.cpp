@@ -117,7 +117,9 @@ int32_t Context::init(int dev)
     // batch kernel already runs
     if (cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming) != cudaSuccess)
+        cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&side_stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ev_side, cudaEventDisableTiming) != cudaSuccess)
         return PBRCM_ERR_CUDA;
     if (cudaMallocHost(&h_one, sizeof(uint32_t)) != cudaSuccess)
         return PBRCM_ERR_OOM;
@@ -241,6 +243,12 @@ Context::~Context()
     if (copy_stream) {
         cudaStreamSynchronize(copy_stream);
         cudaStreamDestroy(copy_stream);
+    }
+    if (ev_side)
+        cudaEventDestroy(ev_side);
+    if (side_stream) {
+        cudaStreamSynchronize(side_stream);
+        cudaStreamDestroy(side_stream);
     }
     if (h_res)
         cudaFreeHost(h_res);

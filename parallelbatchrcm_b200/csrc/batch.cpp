@@ -119,7 +119,8 @@ uint64_t batch_key(const Context& C, const pbrcm_matrix* mats, uint32_t count, c
     for (uint64_t v : {(uint64_t)opt.start, (uint64_t)opt.reverse, (uint64_t)opt.want_bw, (uint64_t)opt.outnodes,
                        (uint64_t)opt.wait_ns, (uint64_t)opt.phantom, (uint64_t)C.batch_pool,
                        (uint64_t)C.cluster_size, (uint64_t)C.cluster_max, (uint64_t)C.cluster_nnz,
-                       (uint64_t)C.solo, (uint64_t)C.batch_solo_kernel, (uint64_t)(uintptr_t)C.d_arena, (uint64_t)(uintptr_t)C.d_jobs,
+                       (uint64_t)C.solo, (uint64_t)C.batch_solo_kernel, (uint64_t)(uint32_t)C.resident_group,
+                       (uint64_t)(uintptr_t)C.d_arena, (uint64_t)(uintptr_t)C.d_jobs,
                        (uint64_t)(uintptr_t)C.d_slots, (uint64_t)(uintptr_t)C.d_bres,
                        (uint64_t)(uintptr_t)C.d_ready, (uint64_t)(uintptr_t)C.d_counter,
                        (uint64_t)(uintptr_t)C.h_bres})
@@ -233,15 +234,49 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
             if (ncl <= 0)
                 nbig = 0;
         }
+        // a batch of at most one matrix per SM: those that fit one CTA's
+        // shared memory go to the shared-memory engine, one CTA each beside
+        // the solo kernel (a small matrix is a chain of levels, at about 1 us
+        // each there against 2 on the solo engine: 96 matrices of 500 to
+        // 5,000 nodes 1.15 -> 1.05 ms; bigger batches need the SMs' throughput).
+        // They come last in the job order.
+        uint32_t nres = 0;
+        size_t res_bytes = 0;
+        int res_g = 0;
+        if (count <= (uint32_t)C.sms && C.resident_group != 0 && C.solo && max_team == 1 && nbig == 0 &&
+            opt.phantom == 0) {
+            uint64_t n_all = 0, nnz_all = 0;
+            for (uint32_t j = 0; j < count; ++j) {
+                n_all += mats[j].n;
+                nnz_all += mats[j].nnz;
+            }
+            res_g = C.resident_group > 0 ? C.resident_group
+                                         : resident_default_group((uint32_t)std::min<uint64_t>(n_all, 0xFFFFFFFFu), nnz_all);
+            auto fits = [&](uint32_t j) {
+                return resident_smem(res_g, mats[j].n, (uint32_t)mats[j].nnz, false) <= (size_t)C.resident_max_smem;
+            };
+            const auto first = std::stable_partition(order.begin(), order.end(), [&](uint32_t j) { return !fits(j); });
+            nres = (uint32_t)(order.end() - first);
+            for (uint32_t q = count - nres; q < count; ++q) {
+                const pbrcm_matrix& m = mats[order[q]];
+                const size_t two = resident_smem(res_g, m.n, (uint32_t)m.nnz, true);
+                res_bytes = std::max(res_bytes, two <= (size_t)C.resident_max_smem
+                                                    ? two
+                                                    : resident_smem(res_g, m.n, (uint32_t)m.nnz, false));
+            }
+        }
+        const uint32_t nsolo = count - nres;  // jobs [nbig, nsolo) take slots
         std::vector<uint32_t> team(count);
         size_t nslots = 0, teamws = 0;
-        for (uint32_t q = nbig; q < count; ++q) {
+        for (uint32_t q = nsolo; q < count; ++q)
+            team[q] = 1;
+        for (uint32_t q = nbig; q < nsolo; ++q) {
             team[q] = team_size(mats[order[q]].nnz, min_nnz, per_cta, max_team);
             nslots += team[q];
             if (team[q] > 1)
                 teamws = align128(teamws + sizeof(GridSync)) + align128(team_words_bytes((int)team[q]));
         }
-        const bool cooperative = nslots > count - nbig;
+        const bool cooperative = nslots > nsolo - nbig;
         use_graph = use_graph && !cooperative;
         // arena layout, in job order (biggest first); every CSR on a 128-byte
         // boundary so that no cache line holds two matrices' data (a
@@ -278,7 +313,7 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
             // for its inverse permutation
             slot[j].e2 = 0;
             slot[j].gvis = 0;
-            if (C.solo && q >= nbig && team[q] == 1 && m.nnz > 0 && m.n <= kSoloMaxNodes) {
+            if (C.solo && q >= nbig && q < nsolo && team[q] == 1 && m.nnz > 0 && m.n <= kSoloMaxNodes) {
                 off = align16(off);
                 slot[j].e2 = off;
                 off += 8 * (size_t)m.nnz;
@@ -344,7 +379,7 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
                 J.words = reinterpret_cast<unsigned long long*>(A + tw);
                 tw = align128(tw + team_words_bytes((int)team[q]));
             }
-            for (uint32_t r = 0; r < team[q]; ++r)
+            for (uint32_t r = 0; r < team[q] && q < nsolo; ++r)
                 C.h_slots[ns++] = BatchSlot{q, r};
         }
         std::memcpy(C.h_jobs, jobs.data(), sizeof(BatchJob) * count);
@@ -379,25 +414,38 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
         }
         bool ok = cudaMemcpyAsync(C.d_jobs, src_jobs, sizeof(BatchJob) * count, cudaMemcpyHostToDevice, st) ==
                       cudaSuccess &&
-                  cudaMemcpyAsync(C.d_slots, src_slots, sizeof(BatchSlot) * nslots, cudaMemcpyHostToDevice, st) ==
-                      cudaSuccess &&
+                  (!nslots || cudaMemcpyAsync(C.d_slots, src_slots, sizeof(BatchSlot) * nslots,
+                                              cudaMemcpyHostToDevice, st) == cudaSuccess) &&
                   (!teamws || cudaMemsetAsync(A + team_off, 0, teamws, st) == cudaSuccess) &&
                   (!nwaves || cudaMemsetAsync(C.d_ready, 0, sizeof(uint32_t) * nwaves, st) == cudaSuccess) &&
                   cudaMemsetAsync(C.d_bres, 0, sizeof(DevResult) * count, st) == cudaSuccess &&
                   cudaMemsetAsync(C.d_counter, 0, 2 * sizeof(uint32_t), st) == cudaSuccess;
         // the copy stream starts once the ready words are zeroed (fork)
+        if (ok && (host || nres))
+            ok = cudaEventRecord(C.ev_fork, st) == cudaSuccess;
         if (ok && host)
-            ok = cudaEventRecord(C.ev_fork, st) == cudaSuccess &&
-                 cudaStreamWaitEvent(C.copy_stream, C.ev_fork, 0) == cudaSuccess;
+            ok = cudaStreamWaitEvent(C.copy_stream, C.ev_fork, 0) == cudaSuccess;
         if (ok && !use_graph)
             ok = cudaEventRecord(C.ev0, st) == cudaSuccess;
+        // the shared-memory engine's CTAs: on device buffers first, since
+        // each wants an SM's shared memory; on host buffers behind the copies
+        // (not waiting for them as the solo kernel does: the launch of a
+        // second kernel may have to wait for the first, and one that waits
+        // for copies not yet issued would never end)
+        auto launch_res = [&](cudaStream_t s) {
+            return launch_batch_resident(res_g, C.d_jobs + nsolo, (int)nres, res_bytes, opt, C.resident_max_smem,
+                                         s) == cudaSuccess;
+        };
+        if (ok && nres && !host)
+            ok = cudaStreamWaitEvent(C.side_stream, C.ev_fork, 0) == cudaSuccess && launch_res(C.side_stream) &&
+                 cudaEventRecord(C.ev_side, C.side_stream) == cudaSuccess;
         if (ok && nbig) {
             Options copt = opt;
             copt.solo_parents = C.cluster_solo_parents;
             copt.solo_edges = C.cluster_solo_edges;
             ok = launch_cluster(v, C.d_jobs, nbig, C.d_slots, (uint32_t)nslots, C.d_counter, copt, opt,
                                 C.cluster_size, ncl, st) == cudaSuccess;
-        } else if (ok) {
+        } else if (ok && nslots) {
             // every job one group's: the solo batch kernel where the shape
             // has one, else the general kernel
             const uint32_t per = (uint32_t)(kPools[v].block / kPools[v].group);
@@ -429,10 +477,14 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
                 ok = ok && cudaMemcpyAsync(C.d_ready + w, C.h_one, sizeof(uint32_t), cudaMemcpyHostToDevice, cs) ==
                                cudaSuccess;
             }
+            if (ok && nres)
+                ok = launch_res(cs);
             // join: nothing after the kernel runs before the copies are done
             ok = ok && cudaEventRecord(C.ev_join, cs) == cudaSuccess &&
                  cudaStreamWaitEvent(st, C.ev_join, 0) == cudaSuccess;
         }
+        if (nres && !host)
+            ok = ok && cudaStreamWaitEvent(st, C.ev_side, 0) == cudaSuccess;
         if (ok && !use_graph)
             ok = cudaEventRecord(C.ev1, st) == cudaSuccess;
         ok = ok && cudaMemcpyAsync(C.h_bres, C.d_bres, sizeof(DevResult) * count, cudaMemcpyDeviceToHost, st) ==
@@ -471,11 +523,12 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
     if (!replayed && !use_graph)
         cudaEventElapsedTime(&dms, C.ev0, C.ev1);
     std::vector<DevResult> res(C.h_bres, C.h_bres + count);
-    // matrices with a hub row rerun on the team path with hub scratch
+    // matrices with a hub row (or one the shared-memory engine's chunks cannot
+    // take) rerun on the team path with hub scratch
     Options topt = make_options(opts, kModeFull);
     apply_team_shape(C, topt);
     for (uint32_t q = 0; q < count; ++q) {
-        if (res[q].status != kNeedHub)
+        if (res[q].status != kNeedHub && res[q].status != kNeedTeam)
             continue;
         const MatrixView& M = jobs[q].M;
         if (!C.ensure_hub(M.nnz))

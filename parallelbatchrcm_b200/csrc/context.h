@@ -102,6 +102,9 @@ struct Context {
     // followed by a copy of *h_one into its ready word d_ready[w]
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    // batches: the shared-memory engine's kernel beside the solo kernel
+    cudaStream_t side_stream = nullptr;
+    cudaEvent_t ev_side = nullptr;
     uint32_t* d_ready = nullptr;
     size_t cap_ready = 0;
     uint32_t* h_one = nullptr;

@@ -73,6 +73,11 @@ size_t resident_smem(int g, uint32_t n, uint32_t nnz, bool spec);
 cudaError_t launch_resident(int g, const uint32_t* rp, const uint32_t* ci, uint32_t n, uint32_t nnz, uint32_t* perm,
                             DevResult* res, const Options& opt, int max_smem, cudaStream_t st);
 
+// The small matrices of a batch (jobs[0 .. count), each fitting `smem`), one
+// CTA each.
+cudaError_t launch_batch_resident(int g, const BatchJob* jobs, int count, size_t smem, const Options& opt,
+                                  int max_smem, cudaStream_t st);
+
 cudaError_t launch_validate(const uint32_t* rp, const uint32_t* ci, uint32_t n, uint32_t nnz, DevResult* res,
                             int sms, cudaStream_t st);
 cudaError_t launch_team(int v, const MatrixView& M, const Options& opt, GridSync* gs, unsigned long long* agg,

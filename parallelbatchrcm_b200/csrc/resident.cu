@@ -420,6 +420,73 @@ __device__ __noinline__ void res_pass_short(ResGroup<G, R>& g, uint32_t start, b
     last_start = lstart;
 }
 
+// One breadth-first pass by the whole CTA, unordered inside a level: what a
+// start-search pass needs while its order does not matter (see the driver).
+// Eight lanes take a parent's row, the exchange of a node's claim word is the
+// whole dedup, a warp appends its children behind one atomic, and a level is
+// one CTA barrier (the ordered passes: three).  tails[L % 3]: children of
+// level L.  The last level ends up in q[last_start .. placed).
+__device__ void res_level_pass(uint32_t n, const uint32_t* rp, const uint32_t* ci, uint32_t* w, uint32_t* q,
+                               uint32_t* tails, uint32_t nnz, DevResult* res, uint32_t start, uint32_t& placed,
+                               uint32_t& nlevels, uint32_t& last_start)
+{
+    const uint32_t tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31u;
+    for (uint32_t i = tid; i < n; i += nthr)
+        w[i] = i == start ? 0u : kUnvisited;
+    if (tid == 0) {
+        q[0] = start;
+        tails[0] = tails[1] = tails[2] = 0;
+    }
+    __syncthreads();
+    const uint32_t qa = saddr(q), wa = saddr(w), rpa = saddr(rp), cia = saddr(ci);
+    uint32_t head = 0, tail = 1, L = 0, slot = 0;
+    while (true) {
+        const uint32_t work = (tail - head) * 8u;
+        for (uint32_t x0 = tid & ~31u; x0 < work; x0 += nthr) {
+            const uint32_t x = x0 + lane;
+            uint32_t k = 0, e = 0;
+            if (x < work) {
+                const uint32_t p = lds(qa + 4 * (head + x / 8u));
+                k = lds(rpa + 4 * p) + (x & 7u);
+                e = lds(rpa + 4 * (p + 1));
+            }
+            while (__any_sync(kFull, k < e)) {
+                uint32_t c = kUnvisited, old = 0;
+                if (k < e && PB_CHECK(res, k < nnz, 632)) {
+                    c = lds(cia + 4 * k);
+                    if (PB_CHECK(res, c < n, 633) && lds(wa + 4 * c) != 0u)
+                        asm volatile("atom.shared.exch.b32 %0, [%1], 0;" : "=r"(old) : "r"(wa + 4 * c) : "memory");
+                }
+                const uint32_t bal = __ballot_sync(kFull, old != 0u);
+                if (bal != 0u) {
+                    uint32_t at = 0;
+                    if (lane == 0)
+                        at = atomicAdd(&tails[slot], (uint32_t)__popc(bal));
+                    at = tail + __shfl_sync(kFull, at, 0) + (uint32_t)__popc(bal & ((1u << lane) - 1u));
+                    if (old != 0u && PB_CHECK(res, at < n, 634))
+                        sts(qa + 4 * at, c);
+                }
+                k += 8;
+            }
+        }
+        __syncthreads();
+        const uint32_t cnt = tails[slot];
+        slot = slot == 2 ? 0 : slot + 1;
+        // the counter of the level after next: last read before this barrier
+        if (tid == 0)
+            tails[slot == 2 ? 0 : slot + 1] = 0;
+        if (cnt == 0)
+            break;
+        head = tail;
+        tail += cnt;
+        ++L;
+    }
+    __syncthreads();
+    placed = tail;
+    nlevels = L + 1;
+    last_start = head;
+}
+
 // CTA-wide reductions (both groups; barrier 0).
 __device__ __forceinline__ unsigned long long cta_max(unsigned long long v, unsigned long long* tmp)
 {
@@ -473,15 +540,15 @@ PBRCM_HD inline size_t res_smem(uint32_t n, uint32_t nnz, bool spec)
 
 // One matrix, one CTA of two groups.  spec: room for the second workspace.
 template <int G, int R>
-__global__ void __launch_bounds__(2 * G, 1)
-    k_reorder_resident(const uint32_t* __restrict__ g_rp, const uint32_t* __restrict__ g_ci, uint32_t n, uint32_t nnz,
-                       uint32_t* perm, DevResult* res, Options opt, uint32_t spec)
+__device__ __forceinline__ void resident_reorder(const uint32_t* __restrict__ g_rp, const uint32_t* __restrict__ g_ci,
+                                                 uint32_t n, uint32_t nnz, uint32_t* perm, DevResult* res,
+                                                 const Options& opt, uint32_t spec)
 {
     constexpr uint32_t EW = (uint32_t)(G * R);
     static_assert(EW == kResidentMaxRow, "every shape chunks kResidentMaxRow edges");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned long long red[2 * G / 32];
-    __shared__ uint32_t ctl[8];
+    __shared__ uint32_t ctl[12];
     using S = ResScratch<G, R>;
     S* scr = reinterpret_cast<S*>(smem_raw);
     uint32_t* rp = reinterpret_cast<uint32_t*>(smem_raw + 2 * sizeof(S));
@@ -553,11 +620,64 @@ __global__ void __launch_bounds__(2 * G, 1)
     // rows of at most 6, 8 or 16 entries: the one-parent-a-thread pass
     const uint32_t row_class = maxdeg <= 6 ? 6u : maxdeg <= 8 ? 8u : maxdeg <= 16 ? 16u : 0u;
     uint32_t lastdist = 0, sorted_from = kUnvisited, s_placed = 0, s_levels = 0;
-    // rounds: group 0 runs a start-search pass while (with spec) group 1
-    // runs the sorted pass from the same start, from the second search on
+    bool repeat = false;  // this round repeats an unordered pass in discovery order
+    // rounds: the first two search passes run unordered by both groups (the
+    // next start -- the last node of minimal valence among the last outnodes
+    // discovered, on the last level -- does not depend on the order when that
+    // level has at most outnodes nodes and one of them alone has the minimal
+    // valence; else the pass is repeated in order); from then on group 0 runs
+    // a start-search pass while (with spec) group 1 runs the sorted pass from
+    // the same start, which the third search pass usually confirms
     while (true) {
         if (!searching && (opt.mode == kModeStartOnly || sorted_from == start))
             break;
+        if (searching && passes < 2 && !repeat) {
+            uint32_t pl, nl, ls;
+            res_level_pass(n, rp, ci, w0, q0, ctl + 8, nnz, res, start, pl, nl, ls);
+            if (read_status(res) != 0)
+                return;
+            if (pl != n) {
+                if (tid == 0)
+                    set_status(res, kErrDisconnected, 0);
+                return;
+            }
+            const uint32_t dist = nl - 1, width = n - ls;
+            if (dist == lastdist) {
+                ++passes;
+                ecc = dist;
+                searching = false;
+                continue;
+            }
+            if (tid < 32) {
+                uint32_t d = kUnvisited, v = 0, same = 0;
+                if (width <= min(opt.outnodes, n - 1))
+                    for (uint32_t i = tid; i < width; i += 32) {
+                        const uint32_t x = q0[ls + i], dx = rp[x + 1] - rp[x];
+                        same = dx < d ? 1u : same + (dx == d ? 1u : 0u);
+                        if (dx < d) {
+                            d = dx;
+                            v = x;
+                        }
+                    }
+                const uint32_t dm = __reduce_min_sync(kFull, d);
+                v = __shfl_sync(kFull, v, __ffs(__ballot_sync(kFull, d == dm)) - 1);
+                const uint32_t count = __reduce_add_sync(kFull, d == dm ? same : 0u);
+                if (tid == 0) {
+                    ctl[5] = v;
+                    ctl[6] = count;
+                }
+            }
+            __syncthreads();
+            repeat = ctl[6] != 1u;
+            if (!repeat) {
+                ++passes;
+                start = ctl[5];
+                lastdist = dist;
+            }
+            __syncthreads();  // ctl is read by all before the next round writes it
+            continue;
+        }
+        repeat = false;
         const bool run_search = searching;
         // (without the second workspace a sorted pass only comes after the search)
         const bool run_sort = opt.mode != kModeStartOnly && (!searching || (spec && passes >= 1));
@@ -712,6 +832,24 @@ __global__ void __launch_bounds__(2 * G, 1)
     }
 }
 
+template <int G, int R>
+__global__ void __launch_bounds__(2 * G, 1)
+    k_reorder_resident(const uint32_t* __restrict__ g_rp, const uint32_t* __restrict__ g_ci, uint32_t n, uint32_t nnz,
+                       uint32_t* perm, DevResult* res, Options opt, uint32_t spec)
+{
+    resident_reorder<G, R>(g_rp, g_ci, n, nnz, perm, res, opt, spec);
+}
+
+// The small matrices of a batch, one CTA each: jobs[0 .. gridDim.x), their
+// CSRs in place.  smem: the launch's dynamic shared memory.
+template <int G, int R>
+__global__ void __launch_bounds__(2 * G, 1) k_batch_resident(const BatchJob* jobs, Options opt, uint32_t smem)
+{
+    const MatrixView M = jobs[blockIdx.x].M;
+    resident_reorder<G, R>(M.rp, M.ci, M.n, M.nnz, M.perm, M.res, opt,
+                           res_smem<G, R>(M.n, M.nnz, true) <= smem ? 1u : 0u);
+}
+
 namespace {
 template <int G, int R>
 struct ResVariant {
@@ -728,6 +866,16 @@ struct ResVariant {
         if (bytes > (size_t)max_smem)
             return cudaErrorInvalidValue;
         k_reorder_resident<G, R><<<1, 2 * G, bytes, st>>>(rp, ci, n, nnz, perm, res, opt, spec ? 1u : 0u);
+        return cudaGetLastError();
+    }
+    static cudaError_t batch(const BatchJob* jobs, int count, size_t bytes, const Options& opt, int max_smem,
+                             cudaStream_t st)
+    {
+        static cudaError_t once = cudaFuncSetAttribute(k_batch_resident<G, R>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+        if (once != cudaSuccess)
+            return once;
+        k_batch_resident<G, R><<<count, 2 * G, bytes, st>>>(jobs, opt, (uint32_t)bytes);
         return cudaGetLastError();
     }
 };
@@ -756,6 +904,13 @@ cudaError_t launch_resident(int g, const uint32_t* rp, const uint32_t* ci, uint3
                             DevResult* res, const Options& opt, int max_smem, cudaStream_t st)
 {
     PBRCM_RES_DISPATCH(g, launch(rp, ci, n, nnz, perm, res, opt, max_smem, st));
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_batch_resident(int g, const BatchJob* jobs, int count, size_t smem, const Options& opt,
+                                  int max_smem, cudaStream_t st)
+{
+    PBRCM_RES_DISPATCH(g, batch(jobs, count, smem, opt, max_smem, st));
     return cudaErrorInvalidValue;
 }
 

@@ -86,12 +86,49 @@ def test_team_search(pbrcm, gpu_ctx_team, built, name):
     assert got == (ref["start"], ref["passes"], ref["ecc"])
 
 
-def test_batch_search(pbrcm, gpu_ctx, built):
+@pytest.fixture(scope="module")
+def solo_ctx(pbrcm, gpu_ctx):
+    """A context whose batches keep every matrix on the solo kernel."""
+    import os
+    old = os.environ.get("PBRCM_RESIDENT_GROUP")
+    os.environ["PBRCM_RESIDENT_GROUP"] = "0"
+    try:
+        ctx = pbrcm.Context(0)
+    finally:
+        if old is None:
+            del os.environ["PBRCM_RESIDENT_GROUP"]
+        else:
+            os.environ["PBRCM_RESIDENT_GROUP"] = old
+    yield ctx
+    ctx.close()
+
+
+@pytest.mark.parametrize("engine", ["default", "solo"])
+@pytest.mark.parametrize("device", [False, True])
+def test_batch_search(pbrcm, gpu_ctx, solo_ctx, built, engine, device):
+    """A batch of fewer matrices than SMs, small ones (shared-memory engine by
+    default) and big ones mixed, from host and from device buffers."""
+    import torch
+    ctx = gpu_ctx if engine == "default" else solo_ctx
     names = list(_cases())
     mats = [built(k)[0] for k in names]
-    perms, res = pbrcm.reorder_batch([(m.row_ptr, m.col_idx) for m in mats], ctx=gpu_ctx)
+    if device:
+        d = [tuple(torch.from_numpy(a.view(np.int32)).cuda() for a in (m.row_ptr, m.col_idx))
+             + (torch.empty(m.n, dtype=torch.int32, device="cuda"),) for m in mats]
+        res = pbrcm.reorder_batch_device(d, ctx=ctx)
+        perms = [x[2].cpu().numpy().view(np.uint32) for x in d]
+    else:
+        perms, res = pbrcm.reorder_batch([(m.row_ptr, m.col_idx) for m in mats], ctx=ctx)
     for k, p, r in zip(names, perms, res):
         _same(p, r, built(k)[1])
+
+
+@pytest.mark.parametrize("name", list(_cases()))
+def test_shared_memory_engine_search(pbrcm, gpu_ctx, built, name):
+    """The single-matrix path's own choice (the shared-memory engine for all
+    but the biggest)."""
+    m, ref = built(name)
+    _same(*pbrcm.reorder(m.row_ptr, m.col_idx, ctx=gpu_ctx), ref)
 
 
 @pytest.mark.parametrize("keep", [1, 4, 40])
