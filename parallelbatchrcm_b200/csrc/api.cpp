@@ -302,13 +302,14 @@ static constexpr int kWideMaxSteps = 1024;
 
 bool Context::run_wide(const MatrixView& M, const Options& opt, cudaStream_t st)
 {
-    const size_t o_tot = 256, o_inv = o_tot + al256(8 * (size_t)wide_ctas);
-    if (!grow(d_wide, cap_wide, o_inv + 4 * (size_t)M.n))
+    const size_t o_tot = 256, o_inv = o_tot + al256(8 * (size_t)wide_ctas), o_maps = o_inv + al256(4 * (size_t)M.n);
+    if (!grow(d_wide, cap_wide, o_maps + wide_maps_bytes(M.n)))
         return false;
+    uint32_t* maps = reinterpret_cast<uint32_t*>(d_wide + o_maps);
     WideState* ws = reinterpret_cast<WideState*>(d_wide);
     unsigned long long* tot = reinterpret_cast<unsigned long long*>(d_wide + o_tot);
     if (cudaMemsetAsync(ws, 0, sizeof(WideState), st) != cudaSuccess ||
-        launch_wide_start(M, opt, ws, sms, st) != cudaSuccess)
+        launch_wide_start(M, opt, ws, maps, sms, st) != cudaSuccess)
         return false;
     WideState* hs = reinterpret_cast<WideState*>(h_aux);
     static_assert(sizeof(WideState) <= 64, "the state is read back through the 64-byte pinned words");
@@ -319,7 +320,7 @@ bool Context::run_wide(const MatrixView& M, const Options& opt, cudaStream_t st)
         if (wide_batch_pass && total > 0 && hs->prev_levels > 0)
             batch = std::max(2, (int)hs->prev_levels + 1 - (int)hs->L);
         batch = std::min(batch, kWideMaxSteps - total);
-        if (launch_wide_steps(M, opt, ws, tot, wide_ctas, batch, wide_fused, st) != cudaSuccess ||
+        if (launch_wide_steps(M, opt, ws, tot, maps, wide_ctas, batch, wide_fused, st) != cudaSuccess ||
             cudaMemcpyAsync(hs, ws, sizeof(WideState), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
             return false;

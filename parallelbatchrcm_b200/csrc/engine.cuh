@@ -912,8 +912,11 @@ struct Chunk {
 
     // Finds the child edges of the chunk, compacts them, ranks every
     // parent's children (sorted = by valence, stable; else slot order) and
-    // computes the edge offsets of the ranked children.
-    __device__ Agg collect(bool sorted, bool from_pre = false)
+    // computes the edge offsets of the ranked children.  BITS: vis holds a bit
+    // per node placed by an earlier level (set here for the children): most
+    // columns of a wide level are settled by it, without their node entry.
+    template <bool BITS = false>
+    __device__ Agg collect(bool sorted, bool from_pre = false, uint32_t* vis = nullptr)
     {
         const uint32_t t = gtid<B>(), lane = t & 31u, w = t >> 5;
         const uint32_t m = s.m, Ec = s.Ec;
@@ -948,6 +951,16 @@ struct Chunk {
                     c[r] = ld_ro(M.ci + idx);
             }
         }
+        if (BITS) {
+            uint32_t word[MAXEPT];
+#pragma unroll
+            for (int r = 0; r < MAXEPT; ++r)
+                word[r] = c[r] != kUnvisited && PB_CHECK(M.res, c[r] < M.n, 162) ? vis[c[r] >> 5] : kFull;
+#pragma unroll
+            for (int r = 0; r < MAXEPT; ++r)
+                if ((word[r] >> (c[r] & 31u)) & 1u)
+                    c[r] = kUnvisited;
+        }
         uint4 nd[MAXEPT];
 #pragma unroll
         for (int r = 0; r < MAXEPT; ++r) {
@@ -962,6 +975,8 @@ struct Chunk {
         for (int r = 0; r < MAXEPT; ++r) {
             if (!(c[r] != kUnvisited && c[r] < M.n && nd[r].x == key[r]))
                 c[r] = kUnvisited;
+            else if (BITS)
+                atomicOr(vis + (c[r] >> 5), 1u << (c[r] & 31u));
             const uint32_t bal = __ballot_sync(kFull, c[r] != kUnvisited);
             pos[r] = __popc(bal & ((1u << lane) - 1u));
             if (lane == 0)
@@ -1170,6 +1185,124 @@ struct Chunk {
         uint32_t c[MAXEPT];
         load_cols(c);
         claim_list(first, c, out, C, flush, [](const Agg&) {});
+    }
+
+    // The share [p_beg, p_end) of a level too wide for one chunk a CTA: no
+    // chunks, each warp works on its own (up to 32 parents with 32 U entries
+    // between them at a time, a row of 32 or more entries alone), so that all
+    // its loads are in flight together and nothing waits at a barrier.  The
+    // node entry is read before the claim: on such levels most columns are
+    // claimed already.  Children go behind the CTA's list `out` while there is
+    // room, else straight to the queue (positions P0 + the level's counter).
+    // A 1M-node geometric graph (levels of 2,300 entries a CTA, bound by the
+    // latency of the gathers): 3.7 ms a call in chunks, 1.87 ms so.
+    __device__ void claim_wide(uint32_t first, uint32_t p_beg, uint32_t p_end, const List& out, Agg& C, uint32_t P0,
+                               unsigned long long* counter)
+    {
+        constexpr uint32_t W = B / 32;
+        // entries a lane holds: 8, or what the warps' entry lists leave room
+        // for in so_idx
+        constexpr int U = 4 * EMAX / (W * 64) < 8 ? 4 * EMAX / (W * 64) : 8;
+        const uint32_t t = gtid<B>(), lane = t & 31u, w = t >> 5;
+        const uint32_t lt = (1u << lane) - 1u;
+        uint16_t* const ent = reinterpret_cast<uint16_t*>(s.so_idx) + w * 32 * U;
+        if (t == 0) {
+            s.bcast[2] = 0;     // taken in `out`
+            s.bcast[3] = EMAX;  // entries of `out` without a gap
+            s.bcast[4] = 0;     // sum of their valences
+        }
+        gsync<B>();
+        const uint32_t F = p_end - p_beg, share = (F + W - 1) / W;
+        const uint32_t pe = p_beg + min(F, (w + 1) * share);
+        for (uint32_t p = p_beg + min(F, w * share); p < pe;) {
+            uint2 r = make_uint2(0u, 0u);  // row start, valence
+            if (p + lane < pe && PB_CHECK(M.res, p + lane < M.n, 158)) {
+                const uint4 q = __ldcg(reinterpret_cast<const uint4*>(M.rec) + p + lane);
+                r = make_uint2(q.y, q.z);
+            }
+            uint32_t x = r.y;
+#pragma unroll
+            for (uint32_t o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFull, x, o);
+                x += lane >= o ? y : 0u;
+            }
+            const uint32_t out_of = ~__ballot_sync(kFull, p + lane < pe && r.y < 32u && x <= 32u * U);
+            const uint32_t m = out_of ? (uint32_t)__ffs(out_of) - 1u : 32u;
+            const uint32_t took = max(m, 1u);
+            const uint32_t soff = x - r.y, shift = r.x - soff;
+            const uint32_t E = __shfl_sync(kFull, x, (int)took - 1);
+            __syncwarp();
+            if (lane < m)
+                for (uint32_t k = 0; k < r.y; ++k)
+                    ent[soff + k] = (uint16_t)lane;
+            __syncwarp();
+            for (uint32_t e0 = 0; e0 < E; e0 += 32u * U) {
+                uint32_t c[U];
+                uint4 nd[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t e = e0 + 32u * u + lane;
+                    c[u] = kUnvisited;
+                    if (e0 + 32u * u < E) {
+                        const uint32_t j = m != 0 ? (uint32_t)ent[32u * u + lane] & 31u : 0u;
+                        const uint32_t idx = __shfl_sync(kFull, shift, (int)j) + e;
+                        if (e < E && PB_CHECK(M.res, idx < M.nnz, 159))
+                            c[u] = ld_ro(M.ci + idx);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    nd[u] = make_uint4(kUnvisited, 0u, 0u, 0u);
+                    if (c[u] != kUnvisited && PB_CHECK(M.res, c[u] < M.n, 160))
+                        nd[u] = ld_node(M.node + c[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (nd[u].x < first)
+                        nd[u].x = atomicMax(&M.node[c[u]].claim, base);
+                uint32_t bal[U], q = 0, dsum = 0;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    bal[u] = __ballot_sync(kFull, nd[u].x < first);
+                    q += __popc(bal[u]);
+                    dsum += nd[u].x < first ? nd[u].z : 0u;
+                }
+                if (q == 0)
+                    continue;
+                dsum = __reduce_add_sync(kFull, dsum);
+                uint32_t at = 0;
+                if (lane == 0)
+                    at = atomicAdd(&s.bcast[2], q);
+                at = __shfl_sync(kFull, at, 0);
+                const bool listed = at + q <= (uint32_t)EMAX;
+                if (lane == 0) {
+                    if (listed) {
+                        atomicAdd(&s.bcast[4], dsum);
+                    } else {
+                        atomicMin(&s.bcast[3], at);
+                        at = P0 + (uint32_t)atomicAdd(counter, (unsigned long long)dsum << 32 | q);
+                    }
+                }
+                at = __shfl_sync(kFull, at, 0);
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t i = at + __popc(bal[u] & lt);
+                    if (nd[u].x < first) {
+                        if (listed) {
+                            out.node[i] = c[u];
+                            out.rs[i] = nd[u].y;
+                            out.deg[i] = nd[u].z;
+                        } else if (PB_CHECK(M.res, i < M.n, 161)) {
+                            __stcg(reinterpret_cast<uint4*>(M.rec) + i, make_uint4(c[u], nd[u].y, nd[u].z, 0u));
+                        }
+                    }
+                    at += __popc(bal[u]);
+                }
+            }
+            p += took;
+        }
+        gsync<B>();
+        C = Agg{min(s.bcast[2], s.bcast[3]), s.bcast[4]};
     }
 
     // Writes the first Q entries of a list to queue positions P0..
@@ -1916,11 +2049,16 @@ __device__ bool level_pass(Smem<B, EMAX>& s, const MatrixView& M, Team& team, co
                 arrived = alone;
             }
         } else {
+            const uint32_t p_beg = st.a + (uint32_t)(((uint64_t)F * R) / G);
             const uint32_t p_end = st.a + (uint32_t)(((uint64_t)F * (R + 1)) / G);
-            for (uint32_t p = st.a + (uint32_t)(((uint64_t)F * R) / G); p < p_end;) {
-                p += ch.form(p, p_end);
-                ch.collect_any(first, out, C, flush);
-            }
+            // (a row over EMAX entries wants the whole CTA)
+            if (queue && M.hub == nullptr)
+                ch.claim_wide(first, p_beg, p_end, out, C, st.b, &team.gs->lvl[slot]);
+            else
+                for (uint32_t p = p_beg; p < p_end;) {
+                    p += ch.form(p, p_end);
+                    ch.collect_any(first, out, C, flush);
+                }
         }
         uint32_t cnt = 0, esum = 0;
         bool keep = false;

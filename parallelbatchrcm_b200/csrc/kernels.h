@@ -141,8 +141,11 @@ cudaError_t launch_bw_rows(const uint32_t* rp, const uint32_t* ci, uint32_t n, c
 // most wide_emax() long.
 int wide_ctas_per_sm();
 uint32_t wide_emax();
-cudaError_t launch_wide_start(const MatrixView& M, const Options& opt, WideState* ws, int sms, cudaStream_t st);
-cudaError_t launch_wide_steps(const MatrixView& M, const Options& opt, WideState* ws, unsigned long long* tot,
+// maps: wide_maps_bytes(n) of visited bitmaps, cleared by the start
+size_t wide_maps_bytes(uint32_t n);
+cudaError_t launch_wide_start(const MatrixView& M, const Options& opt, WideState* ws, uint32_t* maps, int sms,
+                              cudaStream_t st);
+cudaError_t launch_wide_steps(const MatrixView& M, const Options& opt, WideState* ws, unsigned long long* tot, uint32_t* maps,
                               int ctas, int steps, bool fused, cudaStream_t st);
 cudaError_t launch_wide_bandwidth(const MatrixView& M, uint32_t* inv, int sms, cudaStream_t st);
 

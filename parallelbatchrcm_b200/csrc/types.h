@@ -149,11 +149,12 @@ struct Options {
 // State of the level-synchronous engine (wide.cu), one per matrix in device
 // memory: the level being expanded and the start-search bookkeeping, advanced
 // by one kernel after every level.
-enum : uint32_t { kWideSearch = 0, kWideFinal = 1, kWideDone = 2 };
+// (kWideTry: a search pass that runs sorted, the result if it confirms)
+enum : uint32_t { kWideSearch = 0, kWideFinal = 1, kWideDone = 2, kWideTry = 3 };
 struct alignas(16) WideState {
     uint32_t a, b, Ka, Kb;       // frontier positions [a, b), its edge ids [Ka, Kb)
     uint32_t L, last_start;      // level index in the pass, first position of the newest level
-    uint32_t phase;              // kWideSearch / kWideFinal / kWideDone
+    uint32_t phase;              // kWideSearch / kWideFinal / kWideDone / kWideTry
     uint32_t base;               // key base of the pass
     uint32_t start, passes, ecc, lastdist;
     uint32_t pid;                // pass number in the claim key space
