@@ -295,7 +295,7 @@ __device__ __forceinline__ void block_reduce_sum2(unsigned long long& a, unsigne
 }
 
 // Level state of one pass, the same in every CTA of a team.
-constexpr int kTeamShared = 14;  // group-shared ints a team needs (Team::sh)
+constexpr int kTeamShared = 15;  // group-shared ints a team needs (Team::sh)
 
 struct LevelState {
     uint32_t a, b;     // frontier positions [a, b)
@@ -563,17 +563,21 @@ struct Team {
     }
 
     // Second half: the sums over the CTAs before this one (pre) and over
-    // all (all), children in the low and edges in the high 32 bits.
+    // all (all), children in the low and edges in the high 32 bits; over: a
+    // CTA has more than B children or more than emax edges.
     template <int B>
-    __device__ bool ag_collect(uint32_t step, const unsigned long long* agg, unsigned long long& pre,
-                               unsigned long long& all, unsigned long long* red)
+    __device__ bool ag_collect(uint32_t step, const unsigned long long* agg, uint32_t emax, unsigned long long& pre,
+                               unsigned long long& all, bool& over, unsigned long long* red)
     {
         int& s_ok = sh[9];
+        int& s_over = sh[14];
         const uint32_t t = tid;
         pre = 0;
         all = 0;
-        if (t == 0)
+        if (t == 0) {
             s_ok = 1;
+            s_over = 0;
+        }
         gbar();
         for (uint32_t i = t; i < size; i += B) {
             unsigned long long vc, ve;
@@ -595,8 +599,11 @@ struct Team {
             all += v;
             if (i < rank)
                 pre += v;
+            if ((uint32_t)vc > (uint32_t)B || (uint32_t)ve > emax)
+                s_over = 1;
         }
         block_reduce_sum2<B>(pre, all, red);
+        over = s_over != 0;
         return s_ok != 0;
     }
 };
@@ -738,19 +745,23 @@ struct ClusterTeam {
     }
 
     template <int B>
-    __device__ bool ag_collect(uint32_t, const unsigned long long*, unsigned long long& pre, unsigned long long& all,
-                               unsigned long long* red)
+    __device__ bool ag_collect(uint32_t, const unsigned long long*, uint32_t emax, unsigned long long& pre,
+                               unsigned long long& all, bool& over, unsigned long long* red)
     {
         const uint32_t ph = phase & 1u;
         cluster_wait();
         const uint32_t t = tid;
         pre = 0;
         all = 0;
-        if (t == 0)
+        if (t == 0) {
             cs->all_ok = 1;
+            sh[14] = 0;
+        }
         gbar();
         for (uint32_t i = t; i < size; i += B) {
             const ClusterShared* pi = peer(i);
+            if ((uint32_t)pi->ag[ph][0] > (uint32_t)B || (uint32_t)pi->ag[ph][1] > emax)
+                sh[14] = 1;
             const unsigned long long v = (pi->ag[ph][1] << 32) | (pi->ag[ph][0] & 0xFFFFFFFFull);
             if (!pi->ok[ph])
                 atomicAnd(&cs->all_ok, 0u);
@@ -759,6 +770,7 @@ struct ClusterTeam {
                 pre += v;
         }
         block_reduce_sum2<B>(pre, all, red);
+        over = sh[14] != 0;
         ++phase;
         return cs->all_ok != 0;
     }
@@ -1647,12 +1659,14 @@ struct Chunk {
 // One ordered BFS pass from `start` with pass key `base`.  Fills
 // rec[0..placed) and, when write_perm, the output.  Returns false if the team
 // must stop.  nlevels: number of levels; last_start: first position of the
-// last level.
+// last level.  A level of wide_at nodes or more (0: none) hands the matrix to
+// the level-synchronous engine.
 // ---------------------------------------------------------------------------
 template <int B, int EMAX, class TeamT>
 __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, unsigned long long* agg,
-                         uint32_t& step, const Options& opt, uint32_t start, uint32_t base, bool sorted,
-                         bool write_perm, bool reverse, uint32_t& placed, uint32_t& nlevels, uint32_t& last_start)
+                         uint32_t& step, const Options& opt, uint32_t start, uint32_t base, uint32_t wide_at,
+                         bool sorted, bool write_perm, bool reverse, uint32_t& placed, uint32_t& nlevels,
+                         uint32_t& last_start)
 {
     Chunk<B, EMAX> ch{s, M, base};
     const uint32_t t = gtid<B>();
@@ -1690,13 +1704,17 @@ __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, uns
         if (!team.sync(2))
             return false;
     }
+    // own: the next level's share [p_beg, p_end) is this CTA's own children;
+    // carry: they are in shared memory, placed with edge base Kown
+    bool own = false, carry = false;
+    uint32_t p_beg = 0, p_end = 0, Kown = 0;
     while (true) {
         if (solo) {
             // ---- CTA 0 alone: chunk by chunk with running offsets ----------
             if (R == 0) {
                 // carry: the frontier and its adjacency are still in shared
                 // memory from the previous level (it fitted one chunk)
-                bool carry = false;
+                carry = false;
                 bool solo_fail = false;  // stop after handing the gate over
                 while (true) {
                     uint32_t P = st.b, K = st.Kb;
@@ -1781,12 +1799,20 @@ __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, uns
                 break;
             }
             solo = false;
+            carry = false;
             continue;
         }
         // ---- whole team ---------------------------------------------------
-        const uint32_t F = st.b - st.a;
-        const uint32_t p_beg = st.a + (uint32_t)(((uint64_t)F * R) / G);
-        const uint32_t p_end = st.a + (uint32_t)(((uint64_t)F * (R + 1)) / G);
+        // A CTA's children take consecutive positions, so as long as every
+        // CTA's fit one chunk (a share up to that size costs about the same)
+        // each expands its own: they and their columns are still in shared
+        // memory, which saves the level two of its six dependent round trips.
+        // Else the level is split anew into equal runs of the queue.
+        if (!own) {
+            const uint32_t F = st.b - st.a;
+            p_beg = st.a + (uint32_t)(((uint64_t)F * R) / G);
+            p_end = st.a + (uint32_t)(((uint64_t)F * (R + 1)) / G);
+        }
         // A1: collect and count.  A CTA whose parents take several chunks
         // stages each chunk's ranked children (M.stage, at the level-relative
         // edge offset of its first parent: the CTAs' regions are disjoint and
@@ -1797,6 +1823,15 @@ __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, uns
         bool staged = M.stage != nullptr;  // every unit staged (no hub among them)
         uint32_t stage_base = 0;
         uint32_t p = p_beg;
+        if (carry && p < p_end) {
+            ch.form_from_children(Kown);
+            const Agg g = ch.collect(sorted, true);
+            my_cnt = g.cnt;
+            my_esum = g.esum;
+            nunits = 1;
+            p = p_end;
+            gsync<B>();
+        }
         while (p < p_end) {
             const uint32_t used = ch.form(p, p_end);
             if (nunits == 0)
@@ -1825,30 +1860,34 @@ __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, uns
             ch.prefetch();
         // all-gather of the per-CTA totals
         unsigned long long pre = 0, all = 0;
-        if (!team.template ag_collect<B>(step, agg, pre, all, s.gat64))
+        bool over = false;
+        if (!team.template ag_collect<B>(step, agg, (uint32_t)EMAX, pre, all, over, s.gat64))
             return false;
         const uint32_t tot_cnt = (uint32_t)(all & 0xFFFFFFFFull);
         const uint32_t tot_esum = (uint32_t)(all >> 32);
-        if (opt.wide_at != 0 && tot_cnt >= opt.wide_at && base == 2u * M.nnz + 3u &&
-            G == gridDim.x) {
-            // a level this wide in the first pass of the whole team (key base
-            // of pass 1): the level-synchronous engine takes the matrix (every
-            // CTA has the same totals and leaves)
+        // (every CTA has the same totals and leaves)
+        if (wide_at != 0 && tot_cnt >= wide_at) {
             if (R == 0 && t == 0)
                 set_status(M.res, kNeedWide, 0);
             return false;
         }
         uint32_t P = st.b + (uint32_t)(pre & 0xFFFFFFFFull);
         uint32_t K = st.Kb + (uint32_t)(pre >> 32);
+        const uint32_t p_old = p_beg, p_old_end = p_end;
+        own = !over;
+        carry = own && keep && s.npre == my_esum;
+        Kown = K;
+        p_beg = P;
+        p_end = P + my_cnt;
         // A2: place (the only unit is still in shared memory, or all are staged)
         if (keep) {
             ch.place_and_claim(P, K, write_perm, reverse);
         } else if (nunits > 0 && staged) {
             ch.place_staged(stage_base, my_cnt, P, K, write_perm, reverse);
         } else if (nunits > 0) {
-            p = p_beg;
-            while (p < p_end) {
-                const uint32_t used = ch.form(p, p_end);
+            p = p_old;
+            while (p < p_old_end) {
+                const uint32_t used = ch.form(p, p_old_end);
                 if (s.hub) {
                     const uint32_t r0 = s.peb[0] - st.Ka;
                     const uint32_t q = __ldcg(ch.hk1() + r0);
@@ -1881,6 +1920,7 @@ __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, uns
             return false;
         }
         solo = is_solo(st);
+        own = own && !solo;
     }
     placed = st.b;
     nlevels = st.L + 1;
@@ -1906,8 +1946,8 @@ __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, uns
 // queue positions [last_start, placed).
 template <int B, int EMAX>
 __device__ bool level_pass(Smem<B, EMAX>& s, const MatrixView& M, Team& team, const Options& opt, uint32_t start,
-                           uint32_t base, uint32_t first, uint32_t& slot, uint32_t& placed, uint32_t& nlevels,
-                           uint32_t& last_start)
+                           uint32_t base, uint32_t first, uint32_t wide_at, uint32_t& slot, uint32_t& placed,
+                           uint32_t& nlevels, uint32_t& last_start)
 {
     Chunk<B, EMAX> ch{s, M, base};
     using List = typename Chunk<B, EMAX>::List;
@@ -2109,7 +2149,7 @@ __device__ bool level_pass(Smem<B, EMAX>& s, const MatrixView& M, Team& team, co
             slot = slot == 2 ? 0 : slot + 1;
             if (R == 0 && t == 0)
                 __stcg(&team.gs->lvl[slot == 2 ? 0 : slot + 1], 0ull);
-            if (opt.wide_at != 0 && cnt >= opt.wide_at && base == 2u * M.nnz + 3u && G == gridDim.x) {
+            if (wide_at != 0 && cnt >= wide_at) {
                 // a level this wide in the first pass: the level-synchronous
                 // engine takes the matrix (every CTA has the same totals)
                 if (R == 0 && t == 0)
@@ -2130,6 +2170,15 @@ __device__ bool level_pass(Smem<B, EMAX>& s, const MatrixView& M, Team& team, co
     nlevels = st.L + 1;
     last_start = st.last_start;
     return true;
+}
+
+// Stencils wider than 5 and 7 points: more than 8 entries a row, most rows of
+// about the largest valence (random geometric graphs: half of it).  Their
+// breadth-first levels end in a face or an edge, not in a corner, so that a
+// start-search pass always needs discovery order.
+__device__ __forceinline__ bool wide_stencil(uint32_t n, uint32_t nnz, uint32_t maxdeg)
+{
+    return nnz / 8u > n && 4ull * nnz >= 3ull * maxdeg * n;
 }
 
 // Next start of the pseudo-peripheral search (simple_peripheral.cpp:110-127)
@@ -2218,11 +2267,16 @@ __device__ void reorder_matrix(Smem<B, EMAX>& s, const MatrixView& M, TeamT& tea
     // last level has at most outnodes nodes and one of them alone has the
     // minimal valence.  So the search runs unordered (level_pass, about half
     // the time of an ordered level) and only repeats a pass in discovery
-    // order where that fails: never on grids, about a third of the passes of
-    // random geometric graphs.  From the third pass on, which usually
-    // confirms the eccentricity, the search pass is the sorted pass itself
-    // and its order the result if it does.  (Matrices with rows over EMAX and
-    // cluster teams search in discovery order.)
+    // order where that fails: never on 5- and 7-point grids, which end in a
+    // corner, about a third of the passes of random geometric graphs, every
+    // pass on wider stencils (wide_stencil), which therefore begin in discovery
+    // order.  A pass after a repeated one is ordered at once too, until one
+    // would not have had to be (strips of 25-point stencils, 1,001 levels:
+    // 24.2 ms with every pass tried unordered, 18.8 so).  From the third pass
+    // on, which usually confirms the
+    // eccentricity, the search pass is the sorted pass itself and its order
+    // the result if it does.  (Matrices with rows over EMAX and cluster teams
+    // search in discovery order.)
     enum : uint32_t { kLevels, kFifo, kSorted };
     const bool any_order = TeamT::kGrid && G <= 255u && __ldcg(&M.res->maxdeg) <= (uint32_t)EMAX;
     const bool full = opt.mode != kModeStartOnly;
@@ -2236,7 +2290,7 @@ __device__ void reorder_matrix(Smem<B, EMAX>& s, const MatrixView& M, TeamT& tea
     } else if (searching) {
         start = n / 2;
         passes = 1;
-        kind = any_order ? kLevels : kFifo;
+        kind = any_order && !wide_stencil(n, M.nnz, __ldcg(&M.res->maxdeg)) ? kLevels : kFifo;
     }
     while (searching || full) {
         if (pass_id + 1 > pmax) {
@@ -2248,16 +2302,18 @@ __device__ void reorder_matrix(Smem<B, EMAX>& s, const MatrixView& M, TeamT& tea
         }
         ++pass_id;
         const uint32_t base = pass_id * kspan + M.nnz + 1u;
+        const uint32_t wide_at = passes <= 1 && G == gridDim.x ? opt.wide_at : 0u;
         // (one call site of each pass: they are large when inlined)
         if (kind == kLevels) {
             if constexpr (TeamT::kGrid) {
-                if (!level_pass<B, EMAX>(s, M, team, opt, start, base, pass_id * kspan, slot, placed, nlevels,
-                                         last_start))
+                if (!level_pass<B, EMAX>(s, M, team, opt, start, base, pass_id * kspan, wide_at, slot, placed,
+                                         nlevels, last_start))
                     return;
             }
-        } else if (!bfs_pass<B, EMAX>(s, M, team, agg, step, opt, start, base, kind == kSorted, kind == kSorted,
-                                      kind == kSorted && opt.reverse != 0, placed, nlevels, last_start)) {
-            return;
+        } else {
+            if (!bfs_pass<B, EMAX>(s, M, team, agg, step, opt, start, base, wide_at, kind == kSorted,
+                                   kind == kSorted, kind == kSorted && opt.reverse != 0, placed, nlevels, last_start))
+                return;
         }
         if (!searching)
             break;
@@ -2277,23 +2333,19 @@ __device__ void reorder_matrix(Smem<B, EMAX>& s, const MatrixView& M, TeamT& tea
         }
         // the next start (every CTA finds the same)
         const uint32_t width = n - last_start;
-        if (kind == kFifo) {
-            if (t == 0) {
-                s.bcast[0] = next_peripheral_start(M, opt.outnodes, last_start);
-                s.bcast[1] = 1u;
-            }
-        } else if (t < 32) {
+        if (t < 32) {
             uint32_t v = 0, count = 0;
             if (width <= min(opt.outnodes, n - 1))
                 count = unique_min_valence(M, last_start, width, v);
             if (t == 0) {
-                s.bcast[0] = v;
+                s.bcast[0] = kind == kFifo ? next_peripheral_start(M, opt.outnodes, last_start) : v;
                 s.bcast[1] = count == 1u ? 1u : 0u;
             }
         }
         gsync<B>();
         const uint32_t next = s.bcast[0];
-        repeat = s.bcast[1] == 0u;
+        const bool unique = s.bcast[1] != 0u;
+        repeat = kind != kFifo && !unique;
         gsync<B>();
         if (repeat) {
             kind = kFifo;
@@ -2307,7 +2359,7 @@ __device__ void reorder_matrix(Smem<B, EMAX>& s, const MatrixView& M, TeamT& tea
             return;
         }
         ++passes;
-        kind = passes >= 3 && full ? kSorted : any_order ? kLevels : kFifo;
+        kind = passes >= 3 && full ? kSorted : any_order && unique ? kLevels : kFifo;
     }
     if (opt.mode == kModeStartOnly) {
         if (R == 0 && t == 0) {

@@ -620,18 +620,19 @@ __device__ __forceinline__ void resident_reorder(const uint32_t* __restrict__ g_
     // rows of at most 6, 8 or 16 entries: the one-parent-a-thread pass
     const uint32_t row_class = maxdeg <= 6 ? 6u : maxdeg <= 8 ? 8u : maxdeg <= 16 ? 16u : 0u;
     uint32_t lastdist = 0, sorted_from = kUnvisited, s_placed = 0, s_levels = 0;
-    bool repeat = false;  // this round repeats an unordered pass in discovery order
+    bool unordered = !wide_stencil(n, nnz, (uint32_t)maxdeg);
     // rounds: the first two search passes run unordered by both groups (the
     // next start -- the last node of minimal valence among the last outnodes
     // discovered, on the last level -- does not depend on the order when that
     // level has at most outnodes nodes and one of them alone has the minimal
-    // valence; else the pass is repeated in order); from then on group 0 runs
+    // valence; else the pass is repeated in order, and the next one is ordered
+    // at once, as are all of a wide stencil); from then on group 0 runs
     // a start-search pass while (with spec) group 1 runs the sorted pass from
     // the same start, which the third search pass usually confirms
     while (true) {
         if (!searching && (opt.mode == kModeStartOnly || sorted_from == start))
             break;
-        if (searching && passes < 2 && !repeat) {
+        if (searching && passes < 2 && unordered) {
             uint32_t pl, nl, ls;
             res_level_pass(n, rp, ci, w0, q0, ctl + 8, nnz, res, start, pl, nl, ls);
             if (read_status(res) != 0)
@@ -668,8 +669,8 @@ __device__ __forceinline__ void resident_reorder(const uint32_t* __restrict__ g_
                 }
             }
             __syncthreads();
-            repeat = ctl[6] != 1u;
-            if (!repeat) {
+            unordered = ctl[6] == 1u;
+            if (unordered) {
                 ++passes;
                 start = ctl[5];
                 lastdist = dist;
@@ -677,7 +678,6 @@ __device__ __forceinline__ void resident_reorder(const uint32_t* __restrict__ g_
             __syncthreads();  // ctl is read by all before the next round writes it
             continue;
         }
-        repeat = false;
         const bool run_search = searching;
         // (without the second workspace a sorted pass only comes after the search)
         const bool run_sort = opt.mode != kModeStartOnly && (!searching || (spec && passes >= 1));

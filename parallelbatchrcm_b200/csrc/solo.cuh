@@ -668,10 +668,12 @@ __device__ void solo_reorder(SoloSmem<B, EMAX>& s, const MatrixView& M, const ui
         start = n / 2;
     }
     uint32_t lastdist = 0;
+    bool repeat = false;  // this pass repeats the last one in discovery order
+    bool fifo = wide_stencil(n, M.nnz, __ldcg(&M.res->maxdeg));  // this search pass runs in discovery order at once
     while (true) {
         if (!searching && opt.mode == kModeStartOnly)
             break;
-        if (searching)
+        if (searching && !repeat)
             ++passes;
         // a start-search pass has to deliver its level count and the next
         // start, and that start -- the last node of minimal valence among the
@@ -679,17 +681,22 @@ __device__ void solo_reorder(SoloSmem<B, EMAX>& s, const MatrixView& M, const ui
         // (simple_peripheral.cpp:118-127) -- does not depend on the order
         // when the last level has at most outnodes nodes and one of them
         // alone has the minimal valence: the search runs unordered and is
-        // only repeated in order where that fails (never on grids; a third of
-        // the passes of random geometric graphs).  From the third pass on,
+        // only repeated in order where that fails (never on 5- and 7-point
+        // grids; a third of the passes of random geometric graphs; always on
+        // wider stencils, which begin in order; a second pass after one that
+        // needed it is ordered at once).  From the third pass on,
         // which usually confirms the eccentricity, the pass of a sparse
         // matrix is the sorted one itself: the result if it does (444 at once
         // of 100,000 nodes: 2-D grids 12.3 ms against 14.1 with a third
         // unordered pass, 3-D grids 15.3 / 16.6; but random geometric graphs
         // of 11 entries a row, whose third pass confirms less often and whose
         // sorted pass costs two unordered ones, 38.0 / 35.0).
-        const bool sorted = !searching || (passes >= 3 && opt.mode != kModeStartOnly && M.nnz <= 8ull * n);
+        const bool ordered = repeat || fifo;
+        const bool sorted = !searching || (!ordered && passes >= 3 && opt.mode != kModeStartOnly && M.nnz <= 8ull * n);
         if (sorted)
             solo_pass<B, EMAX>(so, start, true, true, opt.reverse != 0, placed, nlevels, last_start);
+        else if (ordered)
+            solo_pass<B, EMAX>(so, start, false, false, false, placed, nlevels, last_start);
         else if (so.gvis)
             solo_level_pass<true, B, EMAX>(so, start, placed, nlevels, last_start);
         else
@@ -704,7 +711,7 @@ __device__ void solo_reorder(SoloSmem<B, EMAX>& s, const MatrixView& M, const ui
             return;
         }
         const uint32_t dist = nlevels - 1;
-        if (dist == lastdist) {
+        if (dist == lastdist && !repeat) {
             ecc = dist;
             searching = false;
             if (sorted)
@@ -717,7 +724,7 @@ __device__ void solo_reorder(SoloSmem<B, EMAX>& s, const MatrixView& M, const ui
             if (t < 32) {
                 uint32_t d = kUnvisited, v = 0, same = 0;
                 for (uint32_t i = t; i < width; i += 32) {
-                    const uint2 r = sorted ? __ldcg(so.q + last_start + i) : s.lbuf[(nlevels - 1) & 1u][i];
+                    const uint2 r = sorted || ordered ? __ldcg(so.q + last_start + i) : s.lbuf[(nlevels - 1) & 1u][i];
                     const uint32_t di = rec_deg(r);
                     same = di < d ? 1u : same + (di == d ? 1u : 0u);
                     if (di < d) {
@@ -736,15 +743,18 @@ __device__ void solo_reorder(SoloSmem<B, EMAX>& s, const MatrixView& M, const ui
             gsync<B>();
             known = s.bcast[1] == 1u;
         }
-        if (!known) {
-            gsync<B>();
-            solo_pass<B, EMAX>(so, start, false, false, false, placed, nlevels, last_start);
-            if (read_status(M.res) != 0)
-                return;
+        gsync<B>();
+        if (!known && !ordered) {
+            repeat = true;
+            continue;
+        }
+        if (ordered) {
             if (t == 0)
                 s.bcast[0] = so.next_start(opt.outnodes, last_start);
             gsync<B>();
         }
+        fifo = !known && passes < 2;
+        repeat = false;
         start = s.bcast[0];
         gsync<B>();
         lastdist = dist;

@@ -116,3 +116,33 @@ def test_rejects_bad_patterns(pbrcm, gpu_ctx):
     with pytest.raises(PbrcmError) as e:
         pbrcm.connect_device(_dev(rp), torch.zeros(1, dtype=torch.int32, device="cuda")[:0], ctx=gpu_ctx)
     assert e.value.status == 7
+
+
+def _band(n, width, first):
+    """Chains of three rows (n rows in all), every row from `first` on with the
+    diagonal and links inside its chain repeated to `width` entries."""
+    rows = []
+    for r in range(n):
+        c = [x for x in range(r // 3 * 3, min(r // 3 * 3 + 3, n)) if abs(x - r) <= 1]
+        rows.append(sorted(c + [r] * max(0, width - len(c))) if r >= first else c)
+    rp = np.concatenate([[0], np.cumsum([len(c) for c in rows])]).astype(np.uint32)
+    return rp, np.concatenate(rows).astype(np.uint32)
+
+
+@pytest.mark.parametrize("n", [31, 32, 33, 63, 64, 65, 257])
+@pytest.mark.parametrize("width", [1, 15, 16, 17, 33])
+def test_row_groups(pbrcm, gpu_ctx, oracle_mod, n, width):
+    """Row counts around the 32 rows a warp takes and rows (of repeated
+    diagonal entries) around the lengths its lanes take together."""
+    _check(pbrcm, gpu_ctx, oracle_mod, *_band(n, width, n // 2))
+
+
+@pytest.mark.parametrize("entry", [(3, 40), (40, 3), (0, 63), (63, 0)])
+def test_one_sided_entry_rejected(pbrcm, gpu_ctx, entry):
+    """An entry without its transpose, above and below the diagonal."""
+    n = 64
+    rows = [sorted({r, max(r - 1, 0), min(r + 1, n - 1)} | ({entry[1]} if r == entry[0] else set()))
+            for r in range(n)]
+    rp = np.concatenate([[0], np.cumsum([len(c) for c in rows])]).astype(np.uint32)
+    with pytest.raises(pbrcm.PbrcmError):
+        _run(pbrcm, gpu_ctx, rp, np.concatenate(rows).astype(np.uint32))

@@ -138,3 +138,25 @@ def test_permute_long_row_on_a_fresh_context(pbrcm, oracle_mod):
             assert np.array_equal(ov, ev)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 2047, 2048, 2049, 4096 * 2048, 4096 * 2048 + 1])
+def test_permute_scan_edges(pbrcm, gpu_ctx, oracle_mod, n):
+    """Row counts around a block of the row-start scan (2,048 rows) and around
+    the 4,096 blocks up to which each adds up the totals before it by itself;
+    a shift by one and the reverse, with the diagonal and a band."""
+    import torch
+    i = torch.arange(n, dtype=torch.int64)
+    deg = 1 + (i % 3 == 0).long() * (i + 1 < n).long()
+    rp = torch.zeros(n + 1, dtype=torch.int64)
+    rp[1:] = deg.cumsum(0)
+    ci = torch.repeat_interleave(i, deg)
+    ci[1:] += (ci[1:] == ci[:-1]).long()
+    rp, ci = rp.int().numpy().view(np.uint32), ci.int().numpy().view(np.uint32)
+    for perm in (((i + 1) % n), n - 1 - i):
+        perm = perm.int().numpy().view(np.uint32)
+        d = [torch.from_numpy(a.view(np.int32)).cuda() for a in (rp, ci, perm)]
+        orp, oci, _, om = pbrcm.permute_device(*d, want_map=True, ctx=gpu_ctx)
+        erp, eci, _, em = oracle_mod.permute_csr(rp, ci, perm)
+        for got, want in ((orp, erp), (oci, eci), (om, em)):
+            assert np.array_equal(got.cpu().numpy().view(np.uint32), want)

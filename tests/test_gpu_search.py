@@ -1,7 +1,7 @@
 """Start-search passes that run unordered inside a level (batch and team
 engines) against the oracle: where the next start is decided without the
-order, where it is not (ties, a last level past the kept nodes) and where
-the unordered pass's shapes have their edges (rows of 31 and 32 entries, 256
+order, where it is not (ties, a last level past the kept nodes, wide
+stencils) and where the unordered pass's shapes have their edges (rows of 31 and 32 entries, 256
 entries a warp, a visited bitmap in global memory)."""
 import numpy as np
 import pytest
@@ -42,6 +42,27 @@ def _hubs(rows, seed):
     return _relabel(n, edges, seed)
 
 
+def _stencil(nx, ny, nz, reach, drop, seed):
+    """A mesh of (2 reach + 1)-wide stencils (9- or 27-point for reach 1);
+    drop: this share of the rows loses its links but a path, which takes the
+    mean valence below the share of the largest that a wide stencil has."""
+    i = np.arange(nx * ny * nz)
+    x, y, z = i % nx, i // nx % ny, i // (nx * ny)
+    rz = reach if nz > 1 else 0
+    edges = [np.stack([i[:-1], i[1:]], 1)]
+    keep = np.random.default_rng(seed).random(i.size) >= drop
+    for dx in range(-reach, reach + 1):
+        for dy in range(-reach, reach + 1):
+            for dz in range(-rz, rz + 1):
+                at = (x + dx, y + dy, z + dz)
+                ok = np.all([(a >= 0) & (a < lim) for a, lim in zip(at, (nx, ny, nz))], axis=0)
+                j = i + dx + dy * nx + dz * nx * ny
+                ok &= j > i
+                ok[ok] &= keep[i[ok]] & keep[j[ok]]
+                edges.append(np.stack([i[ok], j[ok]], 1))
+    return _relabel(i.size, np.concatenate(edges), seed)
+
+
 def _cases():
     from parallelbatchrcm_b200 import gen
     out = {}
@@ -55,6 +76,13 @@ def _cases():
     out["rgg_9001"] = lambda: gen.rgg(9001, kmin=4, kmax=12, seed=6)
     out["rgg_700"] = lambda: gen.rgg(700, kmin=4, kmax=12, seed=8)
     out["grid2d_530x500"] = lambda: gen.grid2d(530, 500, seed=9)  # over 2^18 nodes
+    for drop in (0.0, 0.1, 0.3):  # passes that begin in discovery order, or not
+        out[f"stencil9_60x57_{drop}"] = lambda d=drop: _stencil(60, 57, 1, 1, d, 12)
+        out[f"stencil27_31x29x30_{drop}"] = lambda d=drop: _stencil(31, 29, 30, 1, d, 13)
+    out["stencil25_16x900"] = lambda: _stencil(16, 900, 1, 2, 0.0, 14)
+    out["stencil27_9x8x7"] = lambda: _stencil(9, 8, 7, 1, 0.0, 15)
+    out["random_30000"] = lambda: gen.erdos_renyi(30000, 14, seed=16)  # heavy levels
+    out["random_60000"] = lambda: gen.erdos_renyi(60000, 40, seed=17)  # rows of 32 and more in them
     out["random_5000"] = lambda: gen.erdos_renyi(5000, 14, seed=11)
     return out
 
