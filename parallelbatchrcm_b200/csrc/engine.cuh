@@ -37,11 +37,15 @@
 //            rec[], the node to perm[].
 //   claim:   the placed children claim their own edges for the next level.
 //   A grid team publishes per-CTA (children, valence) totals with a
-//   level-tagged all-gather, places, and meets at a barrier.  Levels with a
-//   small frontier run on CTA 0 alone ("solo") with block barriers only; the
+//   level-tagged all-gather, places, and meets at a barrier; while every
+//   CTA's children fit a chunk each expands its own.  Levels with a small
+//   frontier run on CTA 0 alone ("solo") with block barriers only; the
 //   other CTAs park at a gate until CTA 0 hands a large level back.  Parents
 //   with more than EMAX edges ("hubs") are collected and radix-sorted in
 //   global scratch by one CTA.
+//
+// Start-search passes whose order does not matter (reorder_matrix) run as
+// level_pass instead: a node's first claim of the pass places it.
 //
 // Every wait is bounded by %globaltimer and reports PBRCM_ERR_TIMEOUT.
 // With PBRCM_CHECKS defined, every global index is range-checked and a
@@ -1804,7 +1808,7 @@ __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, uns
         }
         // ---- whole team ---------------------------------------------------
         // A CTA's children take consecutive positions, so as long as every
-        // CTA's fit one chunk (a share up to that size costs about the same)
+        // CTA's fit one chunk and cost no more than an equal share would,
         // each expands its own: they and their columns are still in shared
         // memory, which saves the level two of its six dependent round trips.
         // Else the level is split anew into equal runs of the queue.
@@ -1858,10 +1862,14 @@ __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, uns
         const bool keep = nunits == 1 && !last_hub;
         if (keep)
             ch.prefetch();
-        // all-gather of the per-CTA totals
+        // all-gather of the per-CTA totals (a share costs by rounds of B edges:
+        // own children while they take no more rounds than an equal share:
+        // a 128^3 grid 5.60 ms with any share of one chunk, 5.37 so, 5.53
+        // split anew every level)
+        const uint32_t lim = min((uint32_t)EMAX, ((st.Kb - st.Ka) / G / (uint32_t)B + 1u) * (uint32_t)B);
         unsigned long long pre = 0, all = 0;
         bool over = false;
-        if (!team.template ag_collect<B>(step, agg, (uint32_t)EMAX, pre, all, over, s.gat64))
+        if (!team.template ag_collect<B>(step, agg, lim, pre, all, over, s.gat64))
             return false;
         const uint32_t tot_cnt = (uint32_t)(all & 0xFFFFFFFFull);
         const uint32_t tot_esum = (uint32_t)(all >> 32);
