@@ -166,10 +166,10 @@ int32_t Context::init(int dev)
         resident_group = 0;
     resident_max_smem = (int)prop.sharedMemPerBlockOptin - 2048;  // room for its static shared memory
     // batch / serving shape: built-in defaults (measured on the 4,096-matrix
-    // mixed batch on a B200: the solo batch kernel with three 256-thread
-    // CTAs per SM, 82 ms; 2 x 256 threads per CTA, 86 ms with the solo
-    // kernel and 89-95 ms with the general one; 1 x 512, 102 ms; 2 x 256
-    // with 2,048-edge chunks, 109 ms), or a tuning file written by
+    // mixed batch on a B200: the solo batch kernel with two 256-thread CTAs
+    // per SM, 58.6 ms; three, 66.4 ms; before its unordered search passes 82 ms
+    // against 86 ms for 2 x 256 threads per CTA, 102 ms for 1 x 512 and
+    // 109 ms for 2,048-edge chunks), or a tuning file written by
     // pbrcm_autotune for this device shape and library version
     // (PBRCM_TUNING); a PBRCM_* knob below still overrides a single setting
     pbrcm_tuning tn;

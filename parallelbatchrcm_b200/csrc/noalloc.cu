@@ -28,9 +28,8 @@
 // call this entry point again.
 //
 // Engine: the one-matrix team kernel without the parts that need more
-// scratch -- no speculative final pass beside the start search (second
-// queue-record array), no staging of multi-chunk levels (2 nnz records) and
-// no hub path (rows over kNoAllocMaxValence are refused) -- so it is slower
+// scratch -- no staging of multi-chunk levels (nnz records) and no hub path
+// (rows over kNoAllocMaxValence are refused) -- so it is slower
 // than pbrcm_reorder_device on matrices with wide levels; same result.
 // result->device_ms is the reorder kernel's time from the engine's own
 // %globaltimer stamps.

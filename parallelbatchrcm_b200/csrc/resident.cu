@@ -29,9 +29,11 @@
 // pass).  Five group barriers per chunk, six when sorting; three when every
 // row has at most 16 entries (res_pass_short: one parent per thread).
 //
-// Two groups of G threads: with room for two workspaces, from the second
-// start-search pass on group 1 runs the sorted pass from the same start while
-// group 0 runs the search pass; when the search confirms the eccentricity, the
+// Two groups of G threads.  The first two start-search passes run unordered
+// by both together (res_level_pass) while the next start does not depend on
+// the order.  With room for two workspaces, from then on, and from the second
+// pass on if that is ordered, group 1 runs the sorted pass from the same start
+// while group 0 runs the search pass; when the search confirms the eccentricity, the
 // sorted pass beside it is the answer (one pass less on the critical path).
 // No wait in this kernel spins: the groups meet at CTA barriers only.
 #include "engine.cuh"

@@ -35,6 +35,10 @@
 // by (valence, slot), the writes of the queue records and the permutation,
 // and the visited marks -- four group barriers in the chunk and three where
 // its parents are formed.
+//
+// Start-search passes whose order does not matter run as solo_level_pass
+// instead: no dedup table, no ranks, the first test-and-set of a node's
+// visited bit places it.
 #pragma once
 
 #include "engine.cuh"
