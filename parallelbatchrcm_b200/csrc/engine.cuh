@@ -2099,8 +2099,7 @@ __device__ bool level_pass(Smem<B, EMAX>& s, const MatrixView& M, Team& team, co
         } else {
             const uint32_t p_beg = st.a + (uint32_t)(((uint64_t)F * R) / G);
             const uint32_t p_end = st.a + (uint32_t)(((uint64_t)F * (R + 1)) / G);
-            // (a row over EMAX entries wants the whole CTA)
-            if (queue && M.hub == nullptr)
+            if (queue)
                 ch.claim_wide(first, p_beg, p_end, out, C, st.b, &team.gs->lvl[slot]);
             else
                 for (uint32_t p = p_beg; p < p_end;) {
