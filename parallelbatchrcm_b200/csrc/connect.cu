@@ -40,6 +40,7 @@
 
 #include <cuda_runtime.h>
 
+#include "entries.h"
 #include "kernels.h"
 #include "types.h"
 
@@ -233,16 +234,17 @@ __global__ void __launch_bounds__(kThreads) k_cc_hook(const uint32_t* __restrict
     for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32 < n; w += nwarps) {
         const uint32_t v0 = (uint32_t)(w * 32);
         const RowTile t(rp, n, nnz, v0);
-        for (uint32_t k0 = t.beg; k0 < t.end; k0 += 32u * U) {
+        for (EntrySteps<U> es(t.beg, t.end); es.more(); es.next()) {
             uint32_t v[U], u[U], ub[U], ue[U];
 #pragma unroll
             for (int i = 0; i < U; ++i) {
-                const uint32_t k = k0 + 32u * i + lane;
+                uint32_t k;
+                const bool in = es.entry(i, lane, k);
                 const uint32_t l = t.lane_of(k);
                 const uint32_t b = __shfl_sync(kFull, t.b, l), e = __shfl_sync(kFull, t.e, l);
                 v[i] = v0 + l;
                 u[i] = v[i];  // nothing to do
-                if (k < t.end) {
+                if (in) {
                     if (k < b || k >= e) {  // only a bad row_ptr leaves k outside every row
                         flags |= kFlagRange;
                     } else {
@@ -378,17 +380,19 @@ __global__ void __launch_bounds__(kThreads) k_connect_copy(const uint32_t* __res
                 nl = row_links(parent, n, minn, v0 + lane, lk);
         }
         const bool links = __any_sync(kFull, nl != 0);
-        for (uint32_t k0 = t.beg; k0 < t.end; k0 += 32u * U) {
+        for (EntrySteps<U> es(t.beg, t.end); es.more(); es.next()) {
             uint32_t c[U], l[U];
 #pragma unroll
             for (int i = 0; i < U; ++i) {
-                const uint32_t k = k0 + 32u * i + lane;
+                uint32_t k;
+                const bool in = es.entry(i, lane, k);
                 l[i] = t.lane_of(k);
-                c[i] = k < t.end ? ci[k] : 0u;
+                c[i] = in ? ci[k] : 0u;
             }
 #pragma unroll
             for (int i = 0; i < U; ++i) {
-                const uint32_t k = k0 + 32u * i + lane;
+                uint32_t k;
+                const bool in = es.entry(i, lane, k);
                 const uint32_t b = __shfl_sync(kFull, t.b, l[i]), e = __shfl_sync(kFull, t.e, l[i]);
                 uint64_t at = (uint64_t)__shfl_sync(kFull, ob, l[i]) + (k - b);
                 if (links) {
@@ -396,7 +400,7 @@ __global__ void __launch_bounds__(kThreads) k_connect_copy(const uint32_t* __res
                     const uint32_t l0 = __shfl_sync(kFull, lk[0], l[i]), l1 = __shfl_sync(kFull, lk[1], l[i]);
                     at += (ln > 0 && l0 < c[i] ? 1 : 0) + (ln > 1 && l1 < c[i] ? 1 : 0);
                 }
-                if (k < t.end && k >= b && k < e && at < cap)
+                if (in && k >= b && k < e && at < cap)
                     out_ci[at] = c[i];
             }
         }

@@ -4,11 +4,7 @@
 #include <cstddef>
 #include <cstdint>
 
-#if defined(__CUDACC__)
-#define PBRCM_HD __host__ __device__
-#else
-#define PBRCM_HD
-#endif
+#include "hd.h"
 
 namespace pbrcm {
 
