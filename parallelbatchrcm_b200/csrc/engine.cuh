@@ -56,6 +56,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include "search.h"
 #include "types.h"
 
 namespace pbrcm {
@@ -1794,14 +1795,8 @@ __device__ bool bfs_pass(Smem<B, EMAX>& s, const MatrixView& M, TeamT& team, uns
                 if (!team.gate_wait(st))
                     return false;
             }
-            if (st.a == st.b) {
-                // the pass ended during the solo run: every CTA leaves it
-                // together, so that none can still be reading this gate's
-                // state when CTA 0 opens the next one
-                if (G > 1 && !team.sync(8))
-                    return false;
-                break;
-            }
+            if (st.a == st.b)
+                break;  // the pass ended during the solo run
             solo = false;
             carry = false;
             continue;
@@ -2047,9 +2042,6 @@ __device__ bool level_pass(Smem<B, EMAX>& s, const MatrixView& M, Team& team, co
             return false;
         }
         if (st.a == st.b) {
-            // every CTA leaves the pass together (see bfs_pass)
-            if (G > 1 && !team.sync(8))
-                return false;
             placed = st.b;
             nlevels = st.L + 1;
             last_start = st.last_start;
@@ -2322,6 +2314,30 @@ __device__ void reorder_matrix(Smem<B, EMAX>& s, const MatrixView& M, TeamT& tea
                                    kind == kSorted, kind == kSorted && opt.reverse != 0, placed, nlevels, last_start))
                 return;
         }
+        const uint32_t dist = nlevels - 1;
+        const bool confirmed = dist == lastdist && !repeat;
+        uint32_t next = 0;
+        bool unique = false;
+        if (!end_pass(team, [&]() {
+                if (!searching || placed != n || confirmed)
+                    return;
+                // the next start
+                const uint32_t width = n - last_start;
+                if (t < 32) {
+                    uint32_t v = 0, count = 0;
+                    if (width <= min(opt.outnodes, n - 1))
+                        count = unique_min_valence(M, last_start, width, v);
+                    if (t == 0) {
+                        s.bcast[0] = kind == kFifo ? next_peripheral_start(M, opt.outnodes, last_start) : v;
+                        s.bcast[1] = count == 1u ? 1u : 0u;
+                    }
+                }
+                gsync<B>();
+                next = s.bcast[0];
+                unique = s.bcast[1] != 0u;
+                gsync<B>();
+            }))
+            return;
         if (!searching)
             break;
         if (placed != n) {
@@ -2329,8 +2345,7 @@ __device__ void reorder_matrix(Smem<B, EMAX>& s, const MatrixView& M, TeamT& tea
                 set_status(M.res, kErrDisconnected, 0);
             return;
         }
-        const uint32_t dist = nlevels - 1;
-        if (dist == lastdist && !repeat) {
+        if (confirmed) {
             ecc = dist;
             searching = false;
             if (kind == kSorted)
@@ -2338,22 +2353,7 @@ __device__ void reorder_matrix(Smem<B, EMAX>& s, const MatrixView& M, TeamT& tea
             kind = kSorted;  // the sorted pass from the same start comes next
             continue;
         }
-        // the next start (every CTA finds the same)
-        const uint32_t width = n - last_start;
-        if (t < 32) {
-            uint32_t v = 0, count = 0;
-            if (width <= min(opt.outnodes, n - 1))
-                count = unique_min_valence(M, last_start, width, v);
-            if (t == 0) {
-                s.bcast[0] = kind == kFifo ? next_peripheral_start(M, opt.outnodes, last_start) : v;
-                s.bcast[1] = count == 1u ? 1u : 0u;
-            }
-        }
-        gsync<B>();
-        const uint32_t next = s.bcast[0];
-        const bool unique = s.bcast[1] != 0u;
         repeat = kind != kFifo && !unique;
-        gsync<B>();
         if (repeat) {
             kind = kFifo;
             continue;
