@@ -141,8 +141,8 @@ uint64_t batch_key(const Context& C, const pbrcm_matrix* mats, uint32_t count, c
 //    captured as a CUDA graph on its first call and replayed on later calls
 //    with the same buffers, sizes, options and shape (step 1 is then
 //    skipped);
-// 3. finish: wait, rerun matrices with a hub row on the team path, fill the
-//    results.
+// 3. finish: wait, rerun matrices that their engine could not take (on the
+//    solo kernel, or with a hub row on the team path), fill the results.
 int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, const pbrcm_options* opts,
                          pbrcm_result* results, cudaStream_t st, bool host)
 {
@@ -190,6 +190,16 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
         for (uint32_t j = 0; j < count; ++j)
             in_bytes += 4 * ((size_t)mats[j].n + 1) + 4 * (size_t)mats[j].nnz;
     opt.data_wait_ns = opt.wait_ns + (unsigned long long)in_bytes;
+    // the work list (d_slots): every job one group's, the solo batch kernel
+    // where the shape has one, else the general kernel
+    const uint32_t per = (uint32_t)(kPools[v].block / kPools[v].group);
+    auto launch_slots = [&](uint32_t nslots, bool cooperative) {
+        const int smaxc = C.solo && C.batch_solo_kernel && !cooperative ? solo_max_ctas(v, C.sms) : 0;
+        const int ctas = std::max(1, std::min<int>(smaxc > 0 ? smaxc : maxc, (int)((nslots + per - 1) / per)));
+        return (smaxc > 0 ? launch_solo(v, C.d_jobs, C.d_slots, nslots, C.d_counter, opt, ctas, st)
+                          : launch_batch(v, C.d_jobs, C.d_slots, nslots, C.d_counter, opt, ctas, cooperative,
+                                         st)) == cudaSuccess;
+    };
     float dms = 0.f;
     bool replayed = false;
     if (use_graph && C.bgraph.exec && C.bgraph.key == batch_key(C, mats, count, opt, host) &&
@@ -313,7 +323,7 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
             // for its inverse permutation
             slot[j].e2 = 0;
             slot[j].gvis = 0;
-            if (C.solo && q >= nbig && q < nsolo && team[q] == 1 && m.nnz > 0 && m.n <= kSoloMaxNodes) {
+            if (C.solo && q >= nbig && team[q] == 1 && m.nnz > 0 && m.n <= kSoloMaxNodes) {
                 off = align16(off);
                 slot[j].e2 = off;
                 off += 8 * (size_t)m.nnz;
@@ -346,9 +356,9 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
             }
         }
         if (!grow_dev(C.d_arena, C.cap_arena, off) || !grow_dev(C.d_jobs, C.cap_jobs, count) ||
-            !grow_dev(C.d_bres, C.cap_bres, count) || !grow_dev(C.d_slots, C.cap_slots, nslots) ||
+            !grow_dev(C.d_bres, C.cap_bres, count) || !grow_dev(C.d_slots, C.cap_slots, std::max<size_t>(nslots, count)) ||
             !grow_dev(C.d_counter, C.cap_counter, 8) || (nwaves && !grow_dev(C.d_ready, C.cap_ready, nwaves)) ||
-            !grow_pinned(C.h_jobs, C.cap_hjobs, count) || !grow_pinned(C.h_slots, C.cap_hslots, nslots) ||
+            !grow_pinned(C.h_jobs, C.cap_hjobs, count) || !grow_pinned(C.h_slots, C.cap_hslots, std::max<size_t>(nslots, count)) ||
             !grow_pinned(C.h_bres, C.cap_hbres, count))
             return PBRCM_ERR_OOM;
         unsigned char* A = C.d_arena;
@@ -446,14 +456,7 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
             ok = launch_cluster(v, C.d_jobs, nbig, C.d_slots, (uint32_t)nslots, C.d_counter, copt, opt,
                                 C.cluster_size, ncl, st) == cudaSuccess;
         } else if (ok && nslots) {
-            // every job one group's: the solo batch kernel where the shape
-            // has one, else the general kernel
-            const uint32_t per = (uint32_t)(kPools[v].block / kPools[v].group);
-            const int smaxc = C.solo && C.batch_solo_kernel && !cooperative ? solo_max_ctas(v, C.sms) : 0;
-            const int ctas = std::max(1, std::min<int>(smaxc > 0 ? smaxc : maxc, (int)((nslots + per - 1) / per)));
-            ok = (smaxc > 0 ? launch_solo(v, C.d_jobs, C.d_slots, (uint32_t)nslots, C.d_counter, opt, ctas, st)
-                            : launch_batch(v, C.d_jobs, C.d_slots, (uint32_t)nslots, C.d_counter, opt, ctas,
-                                           cooperative, st)) == cudaSuccess;
+            ok = launch_slots((uint32_t)nslots, cooperative);
         }
         if (ok && host) {
             // the inputs, wave by wave, each wave's ready word after its CSRs
@@ -523,8 +526,35 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
     if (!replayed && !use_graph)
         cudaEventElapsedTime(&dms, C.ev0, C.ev1);
     std::vector<DevResult> res(C.h_bres, C.h_bres + count);
-    // matrices with a hub row (or one the shared-memory engine's chunks cannot
-    // take) rerun on the team path with hub scratch
+    auto perm_back = [&](uint32_t q) {
+        return !host || pdirect[order[q]] ||
+               cudaMemcpyAsync(mats[order[q]].perm_out, jobs[q].M.perm, 4 * (size_t)jobs[q].M.n,
+                               cudaMemcpyDeviceToHost, st) == cudaSuccess;
+    };
+    // the shared-memory engine has refused matrices with a row longer than
+    // its chunks: together in one more launch of the solo kernel (96 matrices
+    // of 3,000 nodes with a row of 600 entries: 0.92 ms, 63 one by one on the
+    // team; a single one takes 0.22 ms there)
+    uint32_t nagain = 0;
+    for (uint32_t q = 0; q < count; ++q)
+        if (res[q].status == kNeedTeam)
+            C.h_slots[nagain++] = BatchSlot{q, 0};
+    if (nagain > 1) {
+        if (cudaMemcpyAsync(C.d_slots, C.h_slots, sizeof(BatchSlot) * nagain, cudaMemcpyHostToDevice, st) !=
+                cudaSuccess ||
+            cudaMemsetAsync(C.d_bres, 0, sizeof(DevResult) * count, st) != cudaSuccess ||
+            cudaMemsetAsync(C.d_counter, 0, 2 * sizeof(uint32_t), st) != cudaSuccess || !launch_slots(nagain, false) ||
+            cudaMemcpyAsync(C.h_bres, C.d_bres, sizeof(DevResult) * count, cudaMemcpyDeviceToHost, st) != cudaSuccess)
+            return PBRCM_ERR_CUDA;
+        for (uint32_t i = 0; i < nagain; ++i)
+            if (!perm_back(C.h_slots[i].job))
+                return PBRCM_ERR_CUDA;
+        if (cudaStreamSynchronize(st) != cudaSuccess)
+            return PBRCM_ERR_CUDA;
+        for (uint32_t i = 0; i < nagain; ++i)
+            res[C.h_slots[i].job] = C.h_bres[C.h_slots[i].job];
+    }
+    // matrices with a hub row rerun on the team path with hub scratch
     Options topt = make_options(opts, kModeFull);
     apply_team_shape(C, topt);
     for (uint32_t q = 0; q < count; ++q) {
@@ -541,9 +571,7 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
             launch_validate(M.rp, M.ci, M.n, M.nnz, M.res, C.sms, st) != cudaSuccess ||
             launch_team(C.team_variant, H, topt, C.d_gs, C.d_agg, C.team_ctas, st) != cudaSuccess ||
             cudaMemcpyAsync(&res[q], M.res, sizeof(DevResult), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            (host && !pdirect[order[q]] &&
-             cudaMemcpyAsync(mats[order[q]].perm_out, M.perm, 4 * (size_t)M.n, cudaMemcpyDeviceToHost, st) !=
-                 cudaSuccess) ||
+            !perm_back(q) ||
             cudaStreamSynchronize(st) != cudaSuccess)
             return PBRCM_ERR_CUDA;
     }

@@ -598,7 +598,7 @@ __device__ __forceinline__ void resident_reorder(const uint32_t* __restrict__ g_
     if (tid == 0)
         res->maxdeg = (uint32_t)maxdeg;
     if (maxdeg > EW) {
-        // a row longer than a chunk: the host reruns the matrix on the team
+        // a row longer than a chunk: the host takes the matrix to another engine
         if (tid == 0)
             set_status(res, kNeedTeam, 0);
         return;

@@ -19,7 +19,7 @@ enum : uint32_t {
     kErrCheck = 8,
     kNeedHub = 100,   // internal: relaunch with hub scratch
     kNeedWide = 101,  // internal: the first pass met a wide level; run the level-synchronous engine
-    kNeedTeam = 102,  // internal: the level-synchronous engine cannot take this matrix; run the team
+    kNeedTeam = 102,  // internal: the level-synchronous or shared-memory engine cannot take this matrix; run another
 };
 
 // One record per queue position: node, row start, valence, edge id base.
