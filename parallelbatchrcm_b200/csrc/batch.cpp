@@ -16,7 +16,9 @@
 #include <algorithm>
 #include <chrono>
 #include <cstring>
+#include <functional>
 #include <numeric>
+#include <queue>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -101,6 +103,24 @@ bool is_pinned(const void* p)
 inline void mix(uint64_t& h, uint64_t v)
 {
     h ^= v + 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2);
+}
+
+// The largest sum of entries a group gets when the jobs order[0 .. count)
+// go, in this order, each to the group with the least.
+uint64_t longest_load(const pbrcm_matrix* mats, const std::vector<uint32_t>& order, uint32_t count, uint32_t groups)
+{
+    std::priority_queue<uint64_t, std::vector<uint64_t>, std::greater<uint64_t>> load;
+    uint64_t longest = 0;
+    for (uint32_t q = 0; q < count; ++q) {
+        uint64_t l = mats[order[q]].nnz;
+        if (q >= groups) {
+            l += load.top();
+            load.pop();
+        }
+        load.push(l);
+        longest = std::max(longest, l);
+    }
+    return longest;
 }
 
 // Everything a captured batch depends on: the matrices' buffers and sizes,
@@ -192,11 +212,12 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
     opt.data_wait_ns = opt.wait_ns + (unsigned long long)in_bytes;
     // the work list (d_slots): every job one group's, the solo batch kernel
     // where the shape has one, else the general kernel
+    // (more: its form for more CTAs per SM)
     const uint32_t per = (uint32_t)(kPools[v].block / kPools[v].group);
-    auto launch_slots = [&](uint32_t nslots, bool cooperative) {
-        const int smaxc = C.solo && C.batch_solo_kernel && !cooperative ? solo_max_ctas(v, C.sms) : 0;
+    auto launch_slots = [&](uint32_t nslots, bool cooperative, bool more) {
+        const int smaxc = C.solo && C.batch_solo_kernel && !cooperative ? solo_max_ctas(v, C.sms, more) : 0;
         const int ctas = std::max(1, std::min<int>(smaxc > 0 ? smaxc : maxc, (int)((nslots + per - 1) / per)));
-        return (smaxc > 0 ? launch_solo(v, C.d_jobs, C.d_slots, nslots, C.d_counter, opt, ctas, st)
+        return (smaxc > 0 ? launch_solo(v, C.d_jobs, C.d_slots, nslots, C.d_counter, opt, ctas, st, more)
                           : launch_batch(v, C.d_jobs, C.d_slots, nslots, C.d_counter, opt, ctas, cooperative,
                                          st)) == cudaSuccess;
     };
@@ -456,7 +477,24 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
             ok = launch_cluster(v, C.d_jobs, nbig, C.d_slots, (uint32_t)nslots, C.d_counter, copt, opt,
                                 C.cluster_size, ncl, st) == cudaSuccess;
         } else if (ok && nslots) {
-            ok = launch_slots((uint32_t)nslots, cooperative);
+            // matrices of about one size: the form of the solo kernel that ends
+            // first by the groups' loads (entries as cost).  Two CTAs per SM run
+            // a matrix 1.2-1.4 times as fast as three and move less through L2
+            // (4,096 of mixed sizes up to 200,000 nodes: 58.6 ms with two, 66.4
+            // with three), but leave a round more where three hold all of them
+            // at once: 444 27-point meshes of 7,200 nodes 4.98 ms with two, 3.25
+            // with three; 888 7.69 / 6.31; 592 5.19 / 5.42.
+            bool more = false;
+            const uint32_t two = per * (uint32_t)std::max(0, solo_max_ctas(v, C.sms)),
+                           three = per * (uint32_t)std::max(0, solo_max_ctas(v, C.sms, true));
+            if (!cooperative && two != 0 && three > two && nsolo > two) {
+                uint64_t sum = 0;
+                for (uint32_t q = 0; q < nsolo; ++q)
+                    sum += mats[order[q]].nnz;
+                more = 2 * (uint64_t)nsolo * mats[order[0]].nnz <= 3 * sum &&
+                       13 * longest_load(mats, order, nsolo, three) < 10 * longest_load(mats, order, nsolo, two);
+            }
+            ok = launch_slots((uint32_t)nslots, cooperative, more);
         }
         if (ok && host) {
             // the inputs, wave by wave, each wave's ready word after its CSRs
@@ -543,7 +581,7 @@ int32_t pbrcm::run_batch(Context& C, const pbrcm_matrix* mats, uint32_t count, c
         if (cudaMemcpyAsync(C.d_slots, C.h_slots, sizeof(BatchSlot) * nagain, cudaMemcpyHostToDevice, st) !=
                 cudaSuccess ||
             cudaMemsetAsync(C.d_bres, 0, sizeof(DevResult) * count, st) != cudaSuccess ||
-            cudaMemsetAsync(C.d_counter, 0, 2 * sizeof(uint32_t), st) != cudaSuccess || !launch_slots(nagain, false) ||
+            cudaMemsetAsync(C.d_counter, 0, 2 * sizeof(uint32_t), st) != cudaSuccess || !launch_slots(nagain, false, false) ||
             cudaMemcpyAsync(C.h_bres, C.d_bres, sizeof(DevResult) * count, cudaMemcpyDeviceToHost, st) != cudaSuccess)
             return PBRCM_ERR_CUDA;
         for (uint32_t i = 0; i < nagain; ++i)

@@ -238,17 +238,17 @@ int batch_max_ctas(int p, int sms)
     return p >= 0 && p < kNumPools ? kPoolTable[p]->batch_max_ctas(sms) : 0;
 }
 
-int solo_max_ctas(int p, int sms)
+int solo_max_ctas(int p, int sms, bool more)
 {
-    return p >= 0 && p < kNumPools ? kPoolTable[p]->solo_max_ctas(sms) : 0;
+    return p >= 0 && p < kNumPools ? kPoolTable[p]->solo_max_ctas(sms, more) : 0;
 }
 
 cudaError_t launch_solo(int p, const BatchJob* jobs, const BatchSlot* slots, uint32_t nslots, uint32_t* counter,
-                        const Options& opt, int ctas, cudaStream_t st)
+                        const Options& opt, int ctas, cudaStream_t st, bool more)
 {
     if (p < 0 || p >= kNumPools)
         return cudaErrorInvalidValue;
-    return kPoolTable[p]->solo(jobs, slots, nslots, counter, opt, ctas, st);
+    return kPoolTable[p]->solo(jobs, slots, nslots, counter, opt, ctas, more, st);
 }
 
 cudaError_t launch_team(int v, const MatrixView& M, const Options& opt, GridSync* gs, unsigned long long* agg,

@@ -43,19 +43,20 @@ struct PoolFns {
     cudaError_t (*cluster)(const BatchJob* jobs, uint32_t nbig, const BatchSlot* slots, uint32_t nslots,
                            uint32_t* counters, const Options& copt, const Options& opt, int csize, int nclusters,
                            cudaStream_t st);
-    int (*solo_max_ctas)(int sms);
+    int (*solo_max_ctas)(int sms, bool more);
     cudaError_t (*solo)(const BatchJob* jobs, const BatchSlot* slots, uint32_t nslots, uint32_t* counter,
-                        const Options& opt, int ctas, cudaStream_t st);
+                        const Options& opt, int ctas, bool more, cudaStream_t st);
 };
 
 size_t variant_smem(int v);
 int team_max_ctas(int v, int sms);   // co-resident CTAs of the team kernel
 int batch_max_ctas(int p, int sms);  // co-resident CTAs of pool p's batch kernel
 // Pool p's solo batch kernel (only one-group jobs with edge records, no
-// teams): co-resident CTAs (0: the shape has none) and the launch.
-int solo_max_ctas(int p, int sms);
+// teams): co-resident CTAs (0: the shape has none) and the launch.  more: the
+// kernel compiled for more CTAs per SM, where the shape has one.
+int solo_max_ctas(int p, int sms, bool more = false);
 cudaError_t launch_solo(int p, const BatchJob* jobs, const BatchSlot* slots, uint32_t nslots, uint32_t* counter,
-                        const Options& opt, int ctas, cudaStream_t st);
+                        const Options& opt, int ctas, cudaStream_t st, bool more = false);
 
 // The shared-memory engine (resident.cu): one CTA of two groups of g
 // threads (32, 64, 128 or 256) holds the matrix in shared memory and runs the

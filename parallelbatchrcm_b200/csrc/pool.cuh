@@ -273,8 +273,9 @@ namespace {
 // whole CTAs, EMAX edges per chunk), split into groups of GB threads (GE
 // edges per chunk) for the one-group slots; MINB CTAs per SM (the register
 // bound the kernels are compiled for); the solo batch kernel of the same
-// groups for SMINB CTAs per SM (0: none for this shape).
-template <int B, int EMAX, int GB, int GE, int MINB, int SMINB>
+// groups for SMINB CTAs per SM (0: none for this shape) and, as an
+// alternative, for SMORE (0: none).
+template <int B, int EMAX, int GB, int GE, int MINB, int SMINB, int SMORE>
 struct Pool {
     static_assert(B % GB == 0 && B / GB <= 15, "at most 15 groups (named barriers 1..15) per CTA");
     static size_t batch_smem() { return (size_t)(B / GB) * group_stride<B, GB, GE>(); }
@@ -335,46 +336,57 @@ struct Pool {
         return cudaLaunchKernelEx(&cfg, k_reorder_cluster<B, EMAX, GB, GE, MINB>, jobs, nbig, slots, nslots, counters, copt,
                                   opt);
     }
-    static constexpr bool kSolo = SMINB > 0 && (size_t)(B / GB) * solo_stride<GB, GE>() <= (size_t)226 * 1024;
     static size_t solo_smem() { return (size_t)(B / GB) * solo_stride<GB, GE>(); }
-    static const void* solo_fn()
+    // the solo batch kernel for PER CTAs per SM (0: none)
+    template <int PER>
+    static constexpr bool has_solo()
     {
-        if constexpr (kSolo)
-            return (const void*)k_solo_batch<B, GB, GE, (SMINB > 0 ? SMINB : 1)>;
-        return nullptr;
+        return PER > 0 && (size_t)(B / GB) * solo_stride<GB, GE>() <= (size_t)226 * 1024;
     }
+    template <int PER>
     static cudaError_t solo_prepare()
     {
-        static cudaError_t once = [] {
-            if (!kSolo)
-                return cudaErrorInvalidValue;
-            return cudaFuncSetAttribute(solo_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solo_smem());
-        }();
-        return once;
+        if constexpr (has_solo<PER>()) {
+            static cudaError_t once = cudaFuncSetAttribute(
+                k_solo_batch<B, GB, GE, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solo_smem());
+            return once;
+        }
+        return cudaErrorInvalidValue;
     }
-    static int solo_max_ctas(int sms)
+    template <int PER>
+    static int solo_max(int sms)
     {
-        if (solo_prepare() != cudaSuccess)
-            return 0;
         int nb = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, solo_fn(), B, solo_smem()) != cudaSuccess) {
-            cudaGetLastError();
-            return 0;
+        if constexpr (has_solo<PER>()) {
+            if (solo_prepare<PER>() != cudaSuccess)
+                return 0;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_solo_batch<B, GB, GE, PER>, B, solo_smem()) !=
+                cudaSuccess) {
+                cudaGetLastError();
+                return 0;
+            }
         }
         return nb * sms;
     }
-    static cudaError_t solo(const BatchJob* jobs, const BatchSlot* slots, uint32_t nslots, uint32_t* counter,
-                            const Options& opt, int ctas, cudaStream_t st)
+    static int solo_max_ctas(int sms, bool more) { return more ? solo_max<SMORE>(sms) : solo_max<SMINB>(sms); }
+    template <int PER>
+    static cudaError_t solo_launch(const BatchJob* jobs, const BatchSlot* slots, uint32_t nslots, uint32_t* counter,
+                                   const Options& opt, int ctas, cudaStream_t st)
     {
-        if constexpr (kSolo) {
-            cudaError_t e = solo_prepare();
+        if constexpr (has_solo<PER>()) {
+            cudaError_t e = solo_prepare<PER>();
             if (e != cudaSuccess)
                 return e;
-            k_solo_batch<B, GB, GE, (SMINB > 0 ? SMINB : 1)><<<ctas, B, solo_smem(), st>>>(jobs, slots, nslots,
-                                                                                           counter, opt);
+            k_solo_batch<B, GB, GE, PER><<<ctas, B, solo_smem(), st>>>(jobs, slots, nslots, counter, opt);
             return cudaGetLastError();
         }
         return cudaErrorInvalidValue;
+    }
+    static cudaError_t solo(const BatchJob* jobs, const BatchSlot* slots, uint32_t nslots, uint32_t* counter,
+                            const Options& opt, int ctas, bool more, cudaStream_t st)
+    {
+        return more ? solo_launch<SMORE>(jobs, slots, nslots, counter, opt, ctas, st)
+                    : solo_launch<SMINB>(jobs, slots, nslots, counter, opt, ctas, st);
     }
     static int batch_max_ctas(int sms)
     {
@@ -412,10 +424,14 @@ struct Pool {
 
 }  // namespace pbrcm
 
-#define PBRCM_DEFINE_POOL(IDX, B, EMAX, GB, GE, MINB, SMINB)                                                \
+#define PBRCM_DEFINE_POOL_MORE(IDX, B, EMAX, GB, GE, MINB, SMINB, SMORE)                                    \
     namespace pbrcm {                                                                                       \
     extern const PoolFns kPoolFns##IDX = {                                                                  \
-        &Pool<B, EMAX, GB, GE, MINB, SMINB>::batch_max_ctas, &Pool<B, EMAX, GB, GE, MINB, SMINB>::cluster_max_active, \
-        &Pool<B, EMAX, GB, GE, MINB, SMINB>::batch, &Pool<B, EMAX, GB, GE, MINB, SMINB>::cluster,                    \
-        &Pool<B, EMAX, GB, GE, MINB, SMINB>::solo_max_ctas, &Pool<B, EMAX, GB, GE, MINB, SMINB>::solo};             \
+        &Pool<B, EMAX, GB, GE, MINB, SMINB, SMORE>::batch_max_ctas,                                         \
+        &Pool<B, EMAX, GB, GE, MINB, SMINB, SMORE>::cluster_max_active,                                     \
+        &Pool<B, EMAX, GB, GE, MINB, SMINB, SMORE>::batch, &Pool<B, EMAX, GB, GE, MINB, SMINB, SMORE>::cluster, \
+        &Pool<B, EMAX, GB, GE, MINB, SMINB, SMORE>::solo_max_ctas,                                          \
+        &Pool<B, EMAX, GB, GE, MINB, SMINB, SMORE>::solo};                                                  \
     }
+#define PBRCM_DEFINE_POOL(IDX, B, EMAX, GB, GE, MINB, SMINB) \
+    PBRCM_DEFINE_POOL_MORE(IDX, B, EMAX, GB, GE, MINB, SMINB, 0)
