@@ -510,10 +510,11 @@ int32_t Context::run_permute(const uint32_t* rp, const uint32_t* ci, const void*
     return map_status(h_res->status);
 }
 
-// parent (n) | scan partials | counters
+// parent (n) | scan partials | counters | row groups of many entries
 size_t Context::connect_work_bytes(uint32_t n)
 {
-    return al256(4 * (size_t)n) + al256(4 * (size_t)scan_partials_count(n)) + 256;
+    return al256(4 * (size_t)n) + al256(4 * (size_t)scan_partials_count(n)) + 256 +
+           sizeof(uint2) * connect_tiles_cap(n);
 }
 
 // The loader's connectivity repair into out_*; its kernels check the CSR as
@@ -526,7 +527,8 @@ int32_t Context::run_connect(const uint32_t* rp, const uint32_t* ci, uint32_t n,
     uint32_t* partials = reinterpret_cast<uint32_t*>(work + al256(4 * (size_t)n));
     uint32_t* counters =
         reinterpret_cast<uint32_t*>(work + al256(4 * (size_t)n) + al256(4 * (size_t)scan_partials_count(n)));
-    if (launch_connect(rp, ci, n, (uint32_t)nnz, out_rp, out_ci, cap, parent, partials, counters, sms, st) !=
+    uint2* tiles = reinterpret_cast<uint2*>(counters + 64);
+    if (launch_connect(rp, ci, n, (uint32_t)nnz, out_rp, out_ci, cap, parent, partials, counters, tiles, sms, st) !=
             cudaSuccess ||
         cudaMemcpyAsync(h_aux, counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)

@@ -13,11 +13,13 @@
 // an empty row, which it queues without marking; the host loader of this
 // library and this pass link it like any other component.)
 //
-// Passes (a warp takes 32 rows at a time and deals their entries out to its
-// lanes, so that no entry searches row_ptr for its row; in the hook pass a
-// lane has four entries' chains of dependent loads in flight):
+// Passes (a warp takes 32 rows at a time, or 1,024 entries of them where they
+// have more, and deals the entries out to its lanes, so that no entry searches
+// row_ptr for its row; in the hook pass a lane has four entries' chains of
+// dependent loads in flight):
 //   1. k_cc_init: parent[v] = min(v, first column of row v) (rows are sorted,
-//      so that is the smallest neighbour) and minn; checks the row pointers;
+//      so that is the smallest neighbour) and minn; checks the row pointers
+//      and lists the groups of 32 rows with more than 1,024 entries;
 //      k_cc_flatten: every node under its root in that forest;
 //   2. k_cc_hook: union-find over the entries (u, v), u < v, hooking the
 //      larger root under the smaller with atomicCAS and halving paths on the
@@ -50,9 +52,13 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kInFlight = 4;  // entries a lane of the hook pass works on at once
+// Entries a warp takes at a time at most: row tiles of more are cut into units
+// of this many (a row has as many entries as its node has neighbours: the
+// repair of a star of 2M nodes takes 72 ms with a tile to a warp, 0.24 so).
+constexpr uint32_t kUnit = 1024;
 
 // counters[0] minn, [1] links, [2] check flags, [3] distinct entries left of
-// the diagonal less those right of it
+// the diagonal less those right of it, [4..5] the 64-bit head of the big tiles
 constexpr uint32_t kFlagRange = 1, kFlagUnsorted = 2, kFlagAsym = 4, kFlagDepth = 8;
 
 // Row v's entry range, clamped into [0, nnz] (a bad row_ptr must not send a
@@ -87,6 +93,58 @@ struct RowTile {
         for (uint32_t d = 16; d > 0; d >>= 1)
             l = __shfl_sync(kFull, b, l + d) <= k ? l + d : l;
         return l;
+    }
+};
+
+// The tiles of more than kUnit entries (k_cc_init lists them): list[i] = {tile,
+// units of the tiles before it}; *head = tiles << 32 | units.
+struct BigTiles {
+    uint2* list;
+    uint32_t cap;  // all tiles
+    unsigned long long* head;
+};
+
+// Work item w of the passes over entries: first every tile of 32 rows, without
+// its entries if it is a big one, then the big tiles' units (with good row
+// pointers at most 2^27 tiles and 2^27 + 2^22 units).
+struct Work {
+    uint32_t tiles, items, nbig;
+    const uint2* list;
+    __device__ __forceinline__ explicit Work(const BigTiles& big) : tiles(big.cap), list(big.list)
+    {
+        const unsigned long long h = __ldcg(big.head);
+        nbig = min((uint32_t)(h >> 32), big.cap);
+        items = tiles + (nbig != 0 ? (uint32_t)h : 0u);
+    }
+    // the first row of item w's tile, and for a unit its number in the tile
+    __device__ __forceinline__ uint32_t row_of(uint32_t w, uint32_t& unit) const
+    {
+        unit = 0;
+        if (w < tiles)
+            return w * 32;
+        const uint32_t x = w - tiles;
+        uint32_t lo = 0;  // the last listed tile that begins at or before unit x
+        for (uint32_t len = nbig; len > 1;) {
+            const uint32_t half = len / 2;
+            if (list[lo + half].y <= x)
+                lo += half;
+            len -= half;
+        }
+        unit = x - list[lo].y;
+        return list[lo].x * 32;
+    }
+    // its entries
+    __device__ __forceinline__ void entries(uint32_t w, uint32_t unit, const RowTile& t, uint32_t& kb,
+                                            uint32_t& ke) const
+    {
+        const uint32_t all = t.end - t.beg, at = unit * kUnit;
+        if (w < tiles) {
+            kb = t.beg;
+            ke = all > kUnit ? t.beg : t.end;
+        } else {
+            kb = at < all ? t.beg + at : t.end;
+            ke = t.end - kb > kUnit ? kb + kUnit : t.end;
+        }
     }
 };
 
@@ -176,9 +234,9 @@ __device__ __forceinline__ int row_links(const uint32_t* __restrict__ parent, ui
     return k > 2 ? 2 : k;
 }
 
-__global__ void __launch_bounds__(kThreads) k_cc_init(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
+__global__ void __launch_bounds__(kThreads, 8) k_cc_init(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
                                                       uint32_t n, uint32_t nnz, uint32_t* __restrict__ parent,
-                                                      uint32_t* counters)
+                                                      uint32_t* counters, BigTiles big)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     uint32_t first = kFull, flags = 0;
@@ -189,6 +247,15 @@ __global__ void __launch_bounds__(kThreads) k_cc_init(const uint32_t* __restrict
         if (e0 < b0 || e0 > nnz || (v == 0 && b0 != 0) || (v == n - 1 && e0 != nnz))
             flags |= kFlagRange;
         row_range(rp, v, nnz, b, e);
+        if ((v & 31u) == 0) {  // the tile's entries
+            const uint32_t end = min(max(rp[min(i + 32, (uint64_t)n)], b), nnz);
+            if (end - b > kUnit) {
+                const unsigned long long units = (end - b - 1) / kUnit + 1;
+                const unsigned long long old = atomicAdd(big.head, 1ull << 32 | units);
+                if ((uint32_t)(old >> 32) < big.cap)  // (bad row pointers may list more)
+                    big.list[old >> 32] = make_uint2(v / 32u, (uint32_t)old);
+            }
+        }
         uint32_t p = v;
         if (e > b) {
             first = min(first, v);
@@ -221,7 +288,8 @@ __global__ void __launch_bounds__(kThreads) k_cc_flatten(uint32_t n, uint32_t* p
 }
 
 __global__ void __launch_bounds__(kThreads) k_cc_hook(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
-                                                      uint32_t n, uint32_t nnz, uint32_t* parent, uint32_t* counters)
+                                                      uint32_t n, uint32_t nnz, uint32_t* parent, uint32_t* counters,
+                                                      BigTiles big)
 {
     constexpr int U = kInFlight;
     if (__ldcg(counters + 2) & kFlagRange)
@@ -229,12 +297,15 @@ __global__ void __launch_bounds__(kThreads) k_cc_hook(const uint32_t* __restrict
     const uint32_t lane = threadIdx.x & 31u;
     __shared__ uint2 pair_list[kThreads / 32][32 * U];
     uint2* const list = pair_list[threadIdx.x >> 5];
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const Work work(big);
     uint32_t flags = 0, lower = 0;
-    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32 < n; w += nwarps) {
-        const uint32_t v0 = (uint32_t)(w * 32);
+    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < work.items; w += nwarps) {
+        uint32_t unit, kb, ke;
+        const uint32_t v0 = work.row_of(w, unit);
         const RowTile t(rp, n, nnz, v0);
-        for (EntrySteps<U> es(t.beg, t.end); es.more(); es.next()) {
+        work.entries(w, unit, t, kb, ke);
+        for (EntrySteps<U> es(kb, ke); es.more(); es.next()) {
             uint32_t v[U], u[U], ub[U], ue[U];
 #pragma unroll
             for (int i = 0; i < U; ++i) {
@@ -357,21 +428,24 @@ __global__ void __launch_bounds__(kThreads) k_connect_rowlen(const uint32_t* __r
 // column); a link e_j goes to out_rp[v] + (entries of v below e_j) + j.
 // Links never coincide with an entry (they join different components).
 // Writes past `cap` are dropped (the host reports the size needed).
-__global__ void __launch_bounds__(kThreads) k_connect_copy(const uint32_t* __restrict__ rp,
+__global__ void __launch_bounds__(kThreads, 6) k_connect_copy(const uint32_t* __restrict__ rp,
                                                            const uint32_t* __restrict__ ci, uint32_t n, uint32_t nnz,
                                                            const uint32_t* __restrict__ parent,
                                                            const uint32_t* counters, const uint32_t* __restrict__ out_rp,
-                                                           uint32_t* __restrict__ out_ci, uint64_t cap)
+                                                           uint32_t* __restrict__ out_ci, uint64_t cap, BigTiles big)
 {
     constexpr int U = 4;
     if (__ldcg(counters + 2) != 0)
         return;  // the call fails
     const uint32_t minn = __ldcg(counters);
     const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32 < n; w += nwarps) {
-        const uint32_t v0 = (uint32_t)(w * 32);
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const Work work(big);
+    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < work.items; w += nwarps) {
+        uint32_t unit, kb, ke;
+        const uint32_t v0 = work.row_of(w, unit);
         const RowTile t(rp, n, nnz, v0);
+        work.entries(w, unit, t, kb, ke);
         uint32_t ob = 0, lk[2] = {0, 0};
         int nl = 0;
         if (v0 + (uint64_t)lane < n) {
@@ -380,7 +454,7 @@ __global__ void __launch_bounds__(kThreads) k_connect_copy(const uint32_t* __res
                 nl = row_links(parent, n, minn, v0 + lane, lk);
         }
         const bool links = __any_sync(kFull, nl != 0);
-        for (EntrySteps<U> es(t.beg, t.end); es.more(); es.next()) {
+        for (EntrySteps<U> es(kb, ke); es.more(); es.next()) {
             uint32_t c[U], l[U];
 #pragma unroll
             for (int i = 0; i < U; ++i) {
@@ -404,7 +478,7 @@ __global__ void __launch_bounds__(kThreads) k_connect_copy(const uint32_t* __res
                     out_ci[at] = c[i];
             }
         }
-        for (int j = 0; j < nl; ++j) {
+        for (int j = 0; j < nl && w < work.tiles; ++j) {
             const uint64_t at = (uint64_t)ob + (lower_bound(ci, t.b, t.e, lk[j]) - t.b) + j;
             if (at < cap)
                 out_ci[at] = lk[j];
@@ -414,30 +488,33 @@ __global__ void __launch_bounds__(kThreads) k_connect_copy(const uint32_t* __res
 
 }  // namespace
 
+uint32_t connect_tiles_cap(uint32_t n) { return (uint32_t)(((uint64_t)n + 31) / 32); }
+
 cudaError_t launch_connect(const uint32_t* rp, const uint32_t* ci, uint32_t n, uint32_t nnz, uint32_t* out_rp,
                            uint32_t* out_ci, uint64_t cap, uint32_t* parent, uint32_t* partials, uint32_t* counters,
-                           int sms, cudaStream_t st)
+                           uint2* tiles, int sms, cudaStream_t st)
 {
     const int rows_blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n + kThreads - 1) / kThreads,
                                                                           (uint64_t)sms * 8));
-    // the passes over entries: a warp per 32 rows
-    const int tile_blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n + kThreads - 1) / kThreads,
-                                                                          (uint64_t)sms * 16));
+    // the passes over entries: a warp per 32 rows, or per unit of a big tile
+    const int tile_blocks = (int)std::max<uint64_t>(
+        1, std::min<uint64_t>(((uint64_t)n + kThreads - 1) / kThreads + nnz / (kUnit * (kThreads / 32)),
+                              (uint64_t)sms * 16));
+    const BigTiles big{tiles, connect_tiles_cap(n), reinterpret_cast<unsigned long long*>(counters + 4)};
     cudaError_t e = cudaMemsetAsync(counters, 0xFF, sizeof(uint32_t), st);
     if (e == cudaSuccess)
-        e = cudaMemsetAsync(counters + 1, 0, 3 * sizeof(uint32_t), st);
+        e = cudaMemsetAsync(counters + 1, 0, 5 * sizeof(uint32_t), st);
     if (e != cudaSuccess)
         return e;
-    k_cc_init<<<rows_blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters);
+    k_cc_init<<<rows_blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters, big);
     k_cc_flatten<<<rows_blocks, kThreads, 0, st>>>(n, parent);
     if (nnz > 0)
-        k_cc_hook<<<tile_blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters);
+        k_cc_hook<<<tile_blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters, big);
     k_connect_rowlen<<<rows_blocks, kThreads, 0, st>>>(rp, n, nnz, parent, counters, out_rp);
     e = launch_scan(out_rp + 1, n, partials, st);
     if (e != cudaSuccess)
         return e;
-    k_connect_copy<<<tile_blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters,
-                                                                             out_rp, out_ci, cap);
+    k_connect_copy<<<tile_blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters, out_rp, out_ci, cap, big);
     return cudaGetLastError();
 }
 

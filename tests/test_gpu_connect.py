@@ -146,3 +146,54 @@ def test_one_sided_entry_rejected(pbrcm, gpu_ctx, entry):
     rp = np.concatenate([[0], np.cumsum([len(c) for c in rows])]).astype(np.uint32)
     with pytest.raises(pbrcm.PbrcmError):
         _run(pbrcm, gpu_ctx, rp, np.concatenate(rows).astype(np.uint32))
+
+
+def _hubs_apart(sizes, at, seed):
+    """Stars (hub rows of the given lengths, diagonal included) that are
+    components of their own among single nodes; the hubs' labels begin at
+    `at`, everything else is shuffled."""
+    n = at + sum(sizes) + 40
+    free = np.random.default_rng(seed).permutation(np.concatenate([np.arange(at), np.arange(at + len(sizes), n)]))
+    rows, cols, used = [np.arange(n)], [np.arange(n)], 0
+    for i, s in enumerate(sizes):
+        leaves = free[used:used + s - 1]
+        used += s - 1
+        hub = np.full(s - 1, at + i)
+        rows += [hub, leaves]
+        cols += [leaves, hub]
+    r, c = np.concatenate(rows), np.concatenate(cols)
+    o = np.lexsort((c, r))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))]).astype(np.uint32)
+    return rp, c[o].astype(np.uint32)
+
+
+@pytest.mark.parametrize("sizes", [[993], [992], [994], [1024], [1025], [1026], [2018, 2], [2048], [5000],
+                                   [700, 700, 700, 3000, 50], [1100] * 70])
+@pytest.mark.parametrize("at", [0, 31, 500])
+def test_long_rows(pbrcm, gpu_ctx, oracle_mod, sizes, at):
+    """Groups of 32 rows around the 1,024 entries a warp takes at a time and
+    far beyond, one and many, with links falling into them."""
+    _check(pbrcm, gpu_ctx, oracle_mod, *_hubs_apart(sizes, at, len(sizes) + at))
+
+
+def test_hub_row_is_shared_out(pbrcm, gpu_ctx):
+    """A star takes about as long as a path of as many nodes (72 ms against
+    0.3 when one warp takes the hub's row)."""
+    import time
+    import torch
+    n, best = 1_000_000, {}
+    i = torch.arange(1, n, device="cuda")
+    for name, j in (("star", torch.zeros_like(i)), ("path", i - 1)):
+        p = torch.randperm(n, generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
+        u, v = p[i], p[j]
+        key = torch.sort(torch.cat([u * n + v, v * n + u])).values
+        rp = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+        rp[1:] = torch.bincount(key // n, minlength=n).cumsum(0)
+        rp, ci = rp.int(), (key % n).int()
+        for _ in range(5):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            _, _, links = pbrcm.connect_device(rp, ci, ctx=gpu_ctx)
+            best[name] = min(best.get(name, 1e9), time.perf_counter() - t)
+        assert links == 0
+    assert best["star"] < 10 * best["path"], best
