@@ -2171,15 +2171,6 @@ __device__ bool level_pass(Smem<B, EMAX>& s, const MatrixView& M, Team& team, co
     return true;
 }
 
-// Stencils wider than 5 and 7 points: more than 8 entries a row, most rows of
-// about the largest valence (random geometric graphs: half of it).  Their
-// breadth-first levels end in a face or an edge, not in a corner, so that a
-// start-search pass always needs discovery order.
-__device__ __forceinline__ bool wide_stencil(uint32_t n, uint32_t nnz, uint32_t maxdeg)
-{
-    return nnz / 8u > n && 4ull * nnz >= 3ull * maxdeg * n;
-}
-
 // Next start of the pseudo-peripheral search (simple_peripheral.cpp:110-127)
 // from the ordered BFS just run: among the last min(outnodes, n-1) positions,
 // those on the last level; the last of minimal valence.  Thread 0 computes.

@@ -622,13 +622,13 @@ __device__ __forceinline__ void resident_reorder(const uint32_t* __restrict__ g_
     // rows of at most 6, 8 or 16 entries: the one-parent-a-thread pass
     const uint32_t row_class = maxdeg <= 6 ? 6u : maxdeg <= 8 ? 8u : maxdeg <= 16 ? 16u : 0u;
     uint32_t lastdist = 0, sorted_from = kUnvisited, s_placed = 0, s_levels = 0;
-    bool unordered = !wide_stencil(n, nnz, (uint32_t)maxdeg);
+    bool unordered = !long_rows((uint32_t)maxdeg) && !wide_stencil(n, nnz, (uint32_t)maxdeg);
     // rounds: the first two search passes run unordered by both groups (the
     // next start -- the last node of minimal valence among the last outnodes
     // discovered, on the last level -- does not depend on the order when that
     // level has at most outnodes nodes and one of them alone has the minimal
     // valence; else the pass is repeated in order, and the next one is ordered
-    // at once, as are all of a wide stencil); from then on group 0 runs
+    // at once, as are all of a wide stencil or with long rows); from then on group 0 runs
     // a start-search pass while (with spec) group 1 runs the sorted pass from
     // the same start, which the third search pass usually confirms
     while (true) {

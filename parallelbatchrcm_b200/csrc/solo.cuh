@@ -507,7 +507,8 @@ __device__ __forceinline__ uint32_t or_if(uint32_t* p, uint32_t v, bool on)
 // once a level: each warp takes up to 32 parents at a time, as many as have
 // 256 entries between them, deals their entries out to its lanes in order
 // (entry e = lane + 32 u; ent[e] = parent lane << 5 | slot names its row), and
-// appends the children it marked.  A row of more than 31 entries goes alone.
+// appends the children it marked.  A row of more than kLevelRow entries goes
+// alone.
 // Returns the last level's records in s.lbuf[(nlevels - 1) & 1] (those past
 // CAP in the queue).  GV: the visited bitmap is in global memory.
 template <bool GV, int B, int EMAX>
@@ -558,9 +559,9 @@ __device__ void solo_level_pass(Solo<B, EMAX>& so, uint32_t start, uint32_t& pla
                 const uint32_t y = __shfl_up_sync(kFull, x, o);
                 x += lane >= o ? y : 0u;
             }
-            // the parents taken: the longest prefix of rows of at most 31
+            // the parents taken: the longest prefix of rows of at most kLevelRow
             // entries, 32 U between them; or one longer row
-            const uint32_t bad = ~__ballot_sync(kFull, i < bend && deg < 32u && x <= 32u * U);
+            const uint32_t bad = ~__ballot_sync(kFull, i < bend && deg <= kLevelRow && x <= 32u * U);
             const uint32_t m = bad ? (uint32_t)__ffs(bad) - 1u : 32u;
             const uint32_t took = max(m, 1u);
             const uint32_t soff = x - deg, shift = r.y - soff;
@@ -673,7 +674,8 @@ __device__ void solo_reorder(SoloSmem<B, EMAX>& s, const MatrixView& M, const ui
     }
     uint32_t lastdist = 0;
     bool repeat = false;  // this pass repeats the last one in discovery order
-    bool fifo = wide_stencil(n, M.nnz, __ldcg(&M.res->maxdeg));  // this search pass runs in discovery order at once
+    const uint32_t maxdeg = __ldcg(&M.res->maxdeg);
+    bool fifo = long_rows(maxdeg) || wide_stencil(n, M.nnz, maxdeg);  // this search pass runs in discovery order at once
     while (true) {
         if (!searching && opt.mode == kModeStartOnly)
             break;
@@ -688,15 +690,16 @@ __device__ void solo_reorder(SoloSmem<B, EMAX>& s, const MatrixView& M, const ui
         // only repeated in order where that fails (never on 5- and 7-point
         // grids; a third of the passes of random geometric graphs; always on
         // wider stencils, which begin in order; a second pass after one that
-        // needed it is ordered at once).  From the third pass on,
+        // needed it is ordered at once, and so is every one of a matrix with
+        // long rows, see long_rows).  From the third pass on,
         // which usually confirms the eccentricity, the pass of a sparse
         // matrix is the sorted one itself: the result if it does (444 at once
         // of 100,000 nodes: 2-D grids 12.3 ms against 14.1 with a third
         // unordered pass, 3-D grids 15.3 / 16.6; but random geometric graphs
         // of 11 entries a row, whose third pass confirms less often and whose
         // sorted pass costs two unordered ones, 38.0 / 35.0).
-        const bool ordered = repeat || fifo;
-        const bool sorted = !searching || (!ordered && passes >= 3 && opt.mode != kModeStartOnly && M.nnz <= 8ull * n);
+        const bool sorted = !searching || (!repeat && passes >= 3 && opt.mode != kModeStartOnly && M.nnz <= 8ull * n);
+        const bool ordered = !sorted && (repeat || fifo);
         if (sorted)
             solo_pass<B, EMAX>(so, start, true, true, opt.reverse != 0, placed, nlevels, last_start);
         else if (ordered)
@@ -757,7 +760,7 @@ __device__ void solo_reorder(SoloSmem<B, EMAX>& s, const MatrixView& M, const ui
                 s.bcast[0] = so.next_start(opt.outnodes, last_start);
             gsync<B>();
         }
-        fifo = !known && passes < 2;
+        fifo = long_rows(maxdeg) || (!known && passes < 2);
         repeat = false;
         start = s.bcast[0];
         gsync<B>();
