@@ -168,6 +168,16 @@ def profile_value(name: str, key: str):
 # ---------------------------------------------------------------------------
 # algorithmic bytes of one full reorder (u32 indices)
 # ---------------------------------------------------------------------------
+def search_passes(engine: str, n: int, nnz: int, passes: int) -> int:
+    """Start-search passes of a reorder beside its sorted one (the `passes` of
+    reorder_bytes), of the `passes` the search took: from the third on, the
+    search pass of the team and of the level-synchronous engine is the sorted
+    pass itself, and so is the solo engine's up to 8 entries a row (the
+    shared-memory engine runs a sorted pass beside it)."""
+    sorted_too = engine in ("team", "wide") or (engine == "solo" and nnz <= 8 * n)
+    return passes - 1 if sorted_too and passes >= 3 else passes
+
+
 def reorder_bytes(n: int, nnz: int, passes: int) -> int:
     """Bytes a full reorder must move at least: each start-search BFS pass
     reads row_ptr 4(n+1) and col_idx 4 nnz and writes a visited word 4n; the
@@ -440,7 +450,8 @@ def measure_grid3d(P, ctx, m, args, ws, stream, flush, dev, cpu: bool):
     t_dev = max_over_ranks(ws, sum(ms) / 1e3)
     t_e2e = max_over_ranks(ws, sum(e2e) / 1e3)
     peak, peak_kind = measured_peak()
-    abytes = reorder_bytes(n, nnz, res["peripheral_passes"])
+    searched = search_passes("team", n, nnz, res["peripheral_passes"])
+    abytes = reorder_bytes(n, nnz, searched)
     achieved = abytes / (statistics.mean(ms) / 1e3) / 1e9
     out = {
         "workload": "grid3d_128^3_7pt_rcm", "n": n, "nnz": nnz, "value": ws * args.steps / t_dev,
@@ -451,18 +462,18 @@ def measure_grid3d(P, ctx, m, args, ws, stream, flush, dev, cpu: bool):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": peak_kind, "kernel": "k_reorder_team<256,1024>",
                      "algorithmic_bytes_per_launch": abytes,
-                     "traffic": profile_value("k_reorder_team_grid3d_128.md", "traffic_bytes_per_launch")},
+                     "traffic": profile_value("k_reorder_team_grid3d_128_unordered.md", "traffic_bytes_per_launch")},
         "result": {"start": res["start_node"], "passes": res["peripheral_passes"], "ecc": res["eccentricity"],
                    "levels": res["levels"], "bandwidth": res["bandwidth"], "profile": res["profile"]},
     }
     # the latency view: the reorder is a chain of dependent BFS levels (each
-    # search pass and the final pass walk about `levels` of them; the last
-    # search pass runs beside the final pass), so time per level of that chain
-    # says more than the HBM fraction
-    chain = res["peripheral_passes"] * res["levels"]
+    # search pass and the sorted one, which is the last search pass too when
+    # the search takes three, walk about `levels` of them), so time per level of
+    # that chain says more than the HBM fraction
+    chain = (searched + 1) * res["levels"]
     out["level_chain"] = {"levels": chain, "us_per_level": t_dev * 1e6 / args.steps / max(1, chain),
-                          "what": "passes x levels of the final order (the last search pass runs beside the "
-                                  "final pass); device time per level of that chain"}
+                          "what": "breadth-first passes x levels of the final order; device time per level of "
+                                  "that chain"}
     if cpu:
         try:
             threads = os.cpu_count() or 1
@@ -558,10 +569,11 @@ def run_mixed(args, ws, rank, local, extras: bool = True):
     # roofline of the batch launch: the algorithmic bytes of every matrix's
     # full reorder over the launch's mean event time
     peak, peak_kind = measured_peak()
-    abytes = sum(reorder_bytes(int(rp.shape[0] - 1), int(ci.shape[0]), r["peripheral_passes"])
-                 for (rp, ci), r in zip(mats, res))
+    sizes = [(int(rp.shape[0] - 1), int(ci.shape[0])) for rp, ci in mats]
+    abytes = sum(reorder_bytes(n, nnz, search_passes("solo", n, nnz, r["peripheral_passes"]))
+                 for (n, nnz), r in zip(sizes, res))
     achieved = abytes / (statistics.mean(times) / 1e3) / 1e9
-    traffic = profile_value("k_solo_batch_mixed_batch_4096.md", "traffic_bytes_per_launch")
+    traffic = profile_value("k_solo_batch_mixed_batch_two_per_sm.md", "traffic_bytes_per_launch")
 
     serve = None
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.int32, device=dev)

@@ -323,7 +323,7 @@ struct Team {
     uint32_t target;     // barriers passed so far
     uint32_t mode;       // barrier implementation (see sync)
     uint32_t epoch;      // gate epochs seen
-    uint32_t word = 0;   // level_sync barriers passed
+    uint32_t word = 0;   // barriers of unordered levels passed (level_wait)
     unsigned long long wait_ns;
     DevResult* res;
     // the thread group running this CTA's part (see gtid): its thread 0 is
@@ -1657,9 +1657,6 @@ struct Chunk {
     }
 };
 
-// ---------------------------------------------------------------------------
-// Level state of one pass.
-// ---------------------------------------------------------------------------
 // ---------------------------------------------------------------------------
 // One ordered BFS pass from `start` with pass key `base`.  Fills
 // rec[0..placed) and, when write_perm, the output.  Returns false if the team

@@ -51,7 +51,7 @@ struct alignas(128) GridSync {
     unsigned int heartbeat;
     unsigned int st[14];
     unsigned long long lvl[3];  // unordered passes: (edges << 32 | nodes) of the level being filled, in rotation
-    unsigned long long word[3];  // unordered passes: barrier words (Team::level_sync)
+    unsigned long long word[3];  // unordered passes: barrier words (Team::level_arrive, level_wait)
     unsigned int pad1[4];
 };
 

@@ -22,3 +22,11 @@ def test_profile_traffic_lines():
     team = bw.profile_value("k_reorder_team_grid3d_128.md", "traffic_bytes_per_launch")
     assert batch == 135_000_000_000 and team == 837_455_360
     assert bw.profile_value("no_such_profile.md", "traffic_bytes_per_launch") is None
+
+
+def test_search_passes_beside_the_sorted_one():
+    # (engine, n, nnz, passes the search took) -> passes counted beside the sorted one
+    for args, want in ((("team", 2097152, 14581760, 3), 2), (("team", 100, 2000, 2), 2), (("wide", 10, 90, 4), 3),
+                       (("solo", 1000, 4960, 3), 2), (("solo", 1000, 8001, 3), 3), (("solo", 1000, 4960, 2), 2),
+                       (("resident", 4096, 20224, 3), 3), (("team", 1, 1, 1), 1)):
+        assert bw.search_passes(*args) == want
