@@ -129,8 +129,9 @@ PBRCM_API int32_t pbrcm_reorder(pbrcm_context* ctx, const uint32_t* row_ptr, con
 
 /*
  * One reorder on DEVICE-resident buffers, enqueued on `stream` (a
- * cudaStream_t, NULL = the context's stream); d_perm_out receives n entries.
- * Synchronises the stream before returning so that `result` is filled.
+ * cudaStream_t, NULL = the context's stream, behind what the legacy default
+ * stream holds at the call); d_perm_out receives n entries.  Synchronises the
+ * stream before returning so that `result` is filled.
  */
 PBRCM_API int32_t pbrcm_reorder_device(pbrcm_context* ctx, const uint32_t* d_row_ptr, const uint32_t* d_col_idx,
                              uint32_t n, uint64_t nnz, const pbrcm_options* opts, uint32_t* d_perm_out,
@@ -201,7 +202,8 @@ PBRCM_API int32_t pbrcm_reorder_batch(pbrcm_context* ctx, const pbrcm_matrix* ma
                             const pbrcm_options* opts, pbrcm_result* results);
 
 /* Same on device-resident CSRs and device perm buffers (pointers in `mats`
- * are device pointers; `mats` itself is a host array). */
+ * are device pointers; `mats` itself is a host array); `stream` as for
+ * pbrcm_reorder_device. */
 PBRCM_API int32_t pbrcm_reorder_batch_device(pbrcm_context* ctx, const pbrcm_matrix* mats, uint32_t count,
                                    const pbrcm_options* opts, pbrcm_result* results, void* stream);
 
@@ -362,8 +364,8 @@ PBRCM_API int32_t pbrcm_permute(pbrcm_context* ctx, const uint32_t* row_ptr, con
                                 const void* vals, uint32_t val_bytes, uint32_t n, uint64_t nnz, const uint32_t* perm,
                                 uint32_t* row_ptr_out, uint32_t* col_idx_out, void* vals_out, uint32_t* map_out);
 
-/* The same on device buffers, enqueued on `stream` (a cudaStream_t; NULL =
- * the context's stream), which is synchronised before returning. */
+/* The same on device buffers, enqueued on `stream` (as for
+ * pbrcm_reorder_device), which is synchronised before returning. */
 PBRCM_API int32_t pbrcm_permute_device(pbrcm_context* ctx, const uint32_t* d_row_ptr, const uint32_t* d_col_idx,
                                        const void* d_vals, uint32_t val_bytes, uint32_t n, uint64_t nnz,
                                        const uint32_t* d_perm, uint32_t* d_row_ptr_out, uint32_t* d_col_idx_out,
@@ -386,7 +388,7 @@ PBRCM_API int32_t pbrcm_permute_device(pbrcm_context* ctx, const uint32_t* d_row
  * *links_out (nullable) = the links added.  A connected matrix comes back
  * unchanged.  With cap_nnz_out below *nnz_out the call returns PBRCM_ERR_ARG
  * with *nnz_out set (the output is incomplete; call again with room).
- * Enqueued on `stream` (NULL = the context's stream), synchronised before
+ * Enqueued on `stream` (as for pbrcm_reorder_device), synchronised before
  * returning.
  */
 PBRCM_API int32_t pbrcm_connect_device(pbrcm_context* ctx, const uint32_t* d_row_ptr, const uint32_t* d_col_idx,

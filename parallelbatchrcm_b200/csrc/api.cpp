@@ -119,7 +119,8 @@ int32_t Context::init(int dev)
         cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaStreamCreateWithFlags(&side_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ev_side, cudaEventDisableTiming) != cudaSuccess)
+        cudaEventCreateWithFlags(&ev_side, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ev_in, cudaEventDisableTiming) != cudaSuccess)
         return PBRCM_ERR_CUDA;
     if (cudaMallocHost(&h_one, sizeof(uint32_t)) != cudaSuccess)
         return PBRCM_ERR_OOM;
@@ -244,6 +245,8 @@ Context::~Context()
         cudaStreamSynchronize(copy_stream);
         cudaStreamDestroy(copy_stream);
     }
+    if (ev_in)
+        cudaEventDestroy(ev_in);
     if (ev_side)
         cudaEventDestroy(ev_side);
     if (side_stream) {
@@ -278,6 +281,20 @@ static bool grow(T*& p, size_t& cap, size_t need)
     }
     cap = want;
     return true;
+}
+
+// The stream of a call on device buffers: the caller's, or (NULL) the context's
+// own, behind what the legacy default stream holds at the call -- the kernels
+// and copies that make the buffers, where a caller uses no stream of its own
+// (1-2 us; the context's stream does not wait for it by itself).
+cudaStream_t Context::device_stream(void* callers)
+{
+    if (callers)
+        return static_cast<cudaStream_t>(callers);
+    if (cudaEventRecord(ev_in, cudaStreamLegacy) != cudaSuccess ||
+        cudaStreamWaitEvent(stream, ev_in, 0) != cudaSuccess)
+        cudaGetLastError();
+    return stream;
 }
 
 bool Context::ensure_single(uint32_t n, uint64_t nnz, bool inputs)
@@ -694,7 +711,7 @@ int32_t pbrcm_reorder_device(pbrcm_context* ctx, const uint32_t* d_row_ptr, cons
     if (!C.ensure_single(n, nnz, false))
         return PBRCM_ERR_OOM;
     Options opt = make_options(opts, kModeFull);
-    cudaStream_t st = stream ? (cudaStream_t)stream : C.stream;
+    cudaStream_t st = C.device_stream(stream);
     DevResult r{};
     float dms = 0.f;
     int32_t rc = C.run_single(d_row_ptr, d_col_idx, n, nnz, d_perm_out, opt, st, &r, &dms);
@@ -723,7 +740,7 @@ int32_t pbrcm_permute_device(pbrcm_context* ctx, const uint32_t* d_row_ptr, cons
     Context& C = ctx->ctx;
     if (!grow(C.d_pw, C.cap_pw, Context::permute_work_bytes(n, nnz)))
         return PBRCM_ERR_OOM;
-    cudaStream_t st = stream ? (cudaStream_t)stream : C.stream;
+    cudaStream_t st = C.device_stream(stream);
     return C.run_permute(d_row_ptr, d_col_idx, d_vals, val_bytes, n, nnz, d_perm, d_row_ptr_out, d_col_idx_out,
                          d_vals_out, d_map_out, C.d_pw, st);
 }
@@ -742,7 +759,7 @@ int32_t pbrcm_connect_device(pbrcm_context* ctx, const uint32_t* d_row_ptr, cons
     Context& C = ctx->ctx;
     if (!grow(C.d_pw, C.cap_pw, Context::connect_work_bytes(n)))
         return PBRCM_ERR_OOM;
-    cudaStream_t st = stream ? (cudaStream_t)stream : C.stream;
+    cudaStream_t st = C.device_stream(stream);
     return C.run_connect(d_row_ptr, d_col_idx, n, nnz, d_row_ptr_out, d_col_idx_out, cap_nnz_out, nnz_out, links_out,
                          C.d_pw, st);
 }

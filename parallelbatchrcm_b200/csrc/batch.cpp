@@ -683,8 +683,7 @@ int32_t pbrcm_reorder_batch_device(pbrcm_context* ctx, const pbrcm_matrix* mats,
     {
         std::lock_guard<std::mutex> lk(ctx->ctx.mu);
         cudaSetDevice(ctx->ctx.device);
-        rc = run_batch(ctx->ctx, mats, count, opts, results, stream ? (cudaStream_t)stream : ctx->ctx.stream,
-                       false);
+        rc = run_batch(ctx->ctx, mats, count, opts, results, ctx->ctx.device_stream(stream), false);
     }
     if (ctx_local)
         pbrcm_context_destroy(ctx_local);

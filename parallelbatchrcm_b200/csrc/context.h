@@ -105,6 +105,7 @@ struct Context {
     // batches: the shared-memory engine's kernel beside the solo kernel
     cudaStream_t side_stream = nullptr;
     cudaEvent_t ev_side = nullptr;
+    cudaEvent_t ev_in = nullptr;  // device_stream
     uint32_t* d_ready = nullptr;
     size_t cap_ready = 0;
     uint32_t* h_one = nullptr;
@@ -138,6 +139,7 @@ struct Context {
 
     int32_t init(int dev);
     ~Context();
+    cudaStream_t device_stream(void* callers);
     bool ensure_single(uint32_t n, uint64_t nnz, bool inputs);
     bool ensure_hub(uint64_t nnz);
     int32_t run_permute(const uint32_t* rp, const uint32_t* ci, const void* vals, uint32_t val_bytes, uint32_t n,

@@ -62,19 +62,6 @@ def _ptr(a: np.ndarray):
     return ctypes.c_void_p(a.ctypes.data)
 
 
-def _stream(stream, device=None) -> int:
-    """The cudaStream_t handle of a call on device tensors: `stream`, or
-    torch's current one.  Handle 0, the default stream, means the context's
-    own stream to the C interface, which does not wait for it: what is queued
-    there (the kernels that make the call's tensors) is finished first."""
-    import torch
-
-    s = stream if stream is not None else torch.cuda.current_stream(device)
-    if s.cuda_stream == 0:
-        s.synchronize()
-    return s.cuda_stream
-
-
 def default_options(reverse: bool = True, start: int | None = None, want_bandwidth: bool = True,
                     peripheral_nodes: int = 32, wait_limit_ms: int = 2000, debug_flags: int = 0,
                     stable: bool = True) -> Options:
@@ -152,7 +139,7 @@ def reorder_device(row_ptr_t, col_idx_t, perm_t=None, *, reverse: bool = True, s
         perm_t = torch.empty(n, dtype=torch.int32, device=row_ptr_t.device)
     res = Result()
     o = default_options(reverse=reverse, start=start, want_bandwidth=want_bandwidth, **opt_kw)
-    st = ctypes.c_void_p(_stream(stream))
+    st = ctypes.c_void_p(stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream)
     rc = _lib.lib().pbrcm_reorder_device(_h(ctx), ctypes.c_void_p(row_ptr_t.data_ptr()),
                                          ctypes.c_void_p(col_idx_t.data_ptr()), n, col_idx_t.numel(),
                                          ctypes.byref(o), ctypes.c_void_p(perm_t.data_ptr()), ctypes.byref(res), st)
@@ -329,7 +316,7 @@ def reorder_batch_device(mats: Sequence, *, reverse: bool = True, ctx: Context |
         raise ValueError("a host PreparedBatch goes to reorder_batch")
     res = (Result * pb.count)()
     o = default_options(reverse=reverse, **opt_kw)
-    st = ctypes.c_void_p(_stream(stream))
+    st = ctypes.c_void_p(stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream)
     rc = _lib.lib().pbrcm_reorder_batch_device(_h(ctx), pb.arr, pb.count, ctypes.byref(o), res, st)
     if raise_on_error:
         _check(rc, "pbrcm_reorder_batch_device")
@@ -498,7 +485,7 @@ def permute_device(row_ptr_t, col_idx_t, perm_t, vals_t=None, *, want_map: bool 
     ov = torch.empty(max(nnz, 1), dtype=vals_t.dtype, device=dev) if vals_t is not None else None
     om = torch.empty(max(nnz, 1), dtype=torch.int32, device=dev) if want_map else None
     vb = vals_t.element_size() if vals_t is not None else 0
-    st = _stream(stream, dev)
+    st = stream.cuda_stream if stream is not None else torch.cuda.current_stream(dev).cuda_stream
     _check(_lib.lib().pbrcm_permute_device(
         _h(ctx), row_ptr_t.data_ptr(), col_idx_t.data_ptr(), vals_t.data_ptr() if vals_t is not None else None,
         vb, n, nnz, perm_t.data_ptr(), orp.data_ptr(), oci.data_ptr(), ov.data_ptr() if ov is not None else None,
@@ -520,7 +507,7 @@ def connect_device(row_ptr_t, col_idx_t, *, cap: int | None = None, ctx: Context
     dev = row_ptr_t.device
     orp = torch.empty(n + 1, dtype=torch.int32, device=dev)
     room = cap if cap is not None else nnz + 2 * min(max(n - 1, 0), max(1024, n // 4))
-    st = _stream(stream, dev)
+    st = stream.cuda_stream if stream is not None else torch.cuda.current_stream(dev).cuda_stream
     L = _lib.lib()
     for _ in range(2):
         oci = torch.empty(max(room, 1), dtype=torch.int32, device=dev)
