@@ -535,7 +535,8 @@ size_t Context::connect_work_bytes(uint32_t n)
 }
 
 // The loader's connectivity repair into out_*; its kernels check the CSR as
-// they read it and clamp every row range; one synchronisation of `st`.
+// they read it and clamp every row range; one synchronisation of `st`, two if 32
+// consecutive rows have more than 1,024 entries.
 int32_t Context::run_connect(const uint32_t* rp, const uint32_t* ci, uint32_t n, uint64_t nnz, uint32_t* out_rp,
                              uint32_t* out_ci, uint64_t cap, uint64_t* nnz_out, uint32_t* links_out,
                              unsigned char* work, cudaStream_t st)
@@ -545,10 +546,20 @@ int32_t Context::run_connect(const uint32_t* rp, const uint32_t* ci, uint32_t n,
     uint32_t* counters =
         reinterpret_cast<uint32_t*>(work + al256(4 * (size_t)n) + al256(4 * (size_t)scan_partials_count(n)));
     uint2* tiles = reinterpret_cast<uint2*>(counters + 64);
+    auto finish = [&]() {
+        return cudaMemcpyAsync(h_aux, counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+               cudaStreamSynchronize(st) == cudaSuccess;
+    };
     if (launch_connect(rp, ci, n, (uint32_t)nnz, out_rp, out_ci, cap, parent, partials, counters, tiles, sms, st) !=
             cudaSuccess ||
-        cudaMemcpyAsync(h_aux, counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
+        !finish())
+        return PBRCM_ERR_CUDA;
+    // rows of many entries: the unions and the output behind the first verdict
+    // (30-40 us more for a few million nodes; other patterns pay nothing for it)
+    if (h_aux[2] == kConnectBig &&
+        (launch_connect_big(rp, ci, n, (uint32_t)nnz, out_rp, out_ci, cap, parent, partials, counters, tiles, sms,
+                              st) != cudaSuccess ||
+         !finish()))
         return PBRCM_ERR_CUDA;
     if (h_aux[2] != 0 || h_aux[3] != 0)
         return PBRCM_ERR_ARG;  // bad row pointers or columns, unsorted row or not symmetric

@@ -13,10 +13,11 @@
 // an empty row, which it queues without marking; the host loader of this
 // library and this pass link it like any other component.)
 //
-// Passes (a warp takes 32 rows at a time, or 1,024 entries of them where they
-// have more, and deals the entries out to its lanes, so that no entry searches
-// row_ptr for its row; in the hook pass a lane has four entries' chains of
-// dependent loads in flight):
+// Passes (a warp takes 32 rows at a time and deals their entries out to its
+// lanes, so that no entry searches row_ptr for its row; in the hook pass a
+// lane has four entries' chains of dependent loads in flight; groups of 32 rows
+// with more than 1,024 entries are cut into units of 512, in a second form of
+// passes 2 and 4):
 //   1. k_cc_init: parent[v] = min(v, first column of row v) (rows are sorted,
 //      so that is the smallest neighbour) and minn; checks the row pointers
 //      and lists the groups of 32 rows with more than 1,024 entries;
@@ -52,14 +53,14 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kInFlight = 4;  // entries a lane of the hook pass works on at once
-// Entries a warp takes at a time at most: row tiles of more are cut into units
-// of this many (a row has as many entries as its node has neighbours: the
-// repair of a star of 2M nodes takes 72 ms with a tile to a warp, 0.24 so).
-constexpr uint32_t kUnit = 1024;
+// A tile of more than kBigTile entries is cut into units of kUnit that all warps
+// take (a row has as many entries as its node has neighbours: the repair of a
+// star of 2M nodes takes 72 ms with a tile to a warp, 0.29 so).
+constexpr uint32_t kBigTile = 1024, kUnit = 512;
 
 // counters[0] minn, [1] links, [2] check flags, [3] distinct entries left of
 // the diagonal less those right of it, [4..5] the 64-bit head of the big tiles
-constexpr uint32_t kFlagRange = 1, kFlagUnsorted = 2, kFlagAsym = 4, kFlagDepth = 8;
+constexpr uint32_t kFlagRange = 1, kFlagUnsorted = 2, kFlagAsym = 4, kFlagDepth = 8, kFlagBig = kConnectBig;
 
 // Row v's entry range, clamped into [0, nnz] (a bad row_ptr must not send a
 // kernel out of bounds before the call's verdict is read).
@@ -96,7 +97,7 @@ struct RowTile {
     }
 };
 
-// The tiles of more than kUnit entries (k_cc_init lists them): list[i] = {tile,
+// The tiles of more than kBigTile entries (k_cc_init lists them): list[i] = {tile,
 // units of the tiles before it}; *head = tiles << 32 | units.
 struct BigTiles {
     uint2* list;
@@ -104,49 +105,47 @@ struct BigTiles {
     unsigned long long* head;
 };
 
-// Work item w of the passes over entries: first every tile of 32 rows, without
-// its entries if it is a big one, then the big tiles' units (with good row
-// pointers at most 2^27 tiles and 2^27 + 2^22 units).
-struct Work {
-    uint32_t tiles, items, nbig;
-    const uint2* list;
-    __device__ __forceinline__ explicit Work(const BigTiles& big) : tiles(big.cap), list(big.list)
-    {
-        const unsigned long long h = __ldcg(big.head);
-        nbig = min((uint32_t)(h >> 32), big.cap);
-        items = tiles + (nbig != 0 ? (uint32_t)h : 0u);
+// What a pass over entries works on: visit(v0, t, kb, ke) for entries [kb, ke) of
+// the tile t from row v0 on -- every tile, or (BIG: there are big ones) every
+// other tile, then the big ones' units.  Patterns with big tiles have kernels of
+// their own, launched behind the verdict that there are any (launch_connect_big):
+// with the units in the same kernels an ordinary pattern takes 2-11 % longer
+// (other registers and spills; 1.2M nodes, 4.5M entries: the hook pass 114 us,
+// 118-137 with them).
+template <bool BIG, class Visit>
+__device__ __forceinline__ void for_tiles(const uint32_t* __restrict__ rp, uint32_t n, uint32_t nnz, Visit visit)
+{
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32 < n; w += nwarps) {
+        const uint32_t v0 = (uint32_t)(w * 32);
+        const RowTile t(rp, n, nnz, v0);
+        if (!BIG || t.end - t.beg <= kBigTile)
+            visit(v0, t, t.beg, t.end);
     }
-    // the first row of item w's tile, and for a unit its number in the tile
-    __device__ __forceinline__ uint32_t row_of(uint32_t w, uint32_t& unit) const
-    {
-        unit = 0;
-        if (w < tiles)
-            return w * 32;
-        const uint32_t x = w - tiles;
+}
+
+template <class Visit>
+__device__ __forceinline__ void for_units(const uint32_t* __restrict__ rp, uint32_t n, uint32_t nnz,
+                                          const BigTiles& big, Visit visit)
+{
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const unsigned long long head = __ldcg(big.head);
+    const uint32_t tiles = min((uint32_t)(head >> 32), big.cap), units = tiles != 0 ? (uint32_t)head : 0u;
+    for (uint64_t x = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < units; x += nwarps) {
         uint32_t lo = 0;  // the last listed tile that begins at or before unit x
-        for (uint32_t len = nbig; len > 1;) {
+        for (uint32_t len = tiles; len > 1;) {
             const uint32_t half = len / 2;
-            if (list[lo + half].y <= x)
+            if (big.list[lo + half].y <= x)
                 lo += half;
             len -= half;
         }
-        unit = x - list[lo].y;
-        return list[lo].x * 32;
+        const uint2 at = big.list[lo];
+        const RowTile t(rp, n, nnz, at.x * 32);
+        const uint32_t all = t.end - t.beg, k = ((uint32_t)x - at.y) * kUnit;
+        const uint32_t kb = k < all ? t.beg + k : t.end;
+        visit(at.x * 32, t, kb, t.end - kb > kUnit ? kb + kUnit : t.end);
     }
-    // its entries
-    __device__ __forceinline__ void entries(uint32_t w, uint32_t unit, const RowTile& t, uint32_t& kb,
-                                            uint32_t& ke) const
-    {
-        const uint32_t all = t.end - t.beg, at = unit * kUnit;
-        if (w < tiles) {
-            kb = t.beg;
-            ke = all > kUnit ? t.beg : t.end;
-        } else {
-            kb = at < all ? t.beg + at : t.end;
-            ke = t.end - kb > kUnit ? kb + kUnit : t.end;
-        }
-    }
-};
+}
 
 // First index in ci[b, e) whose column is >= x (a sorted row).
 __device__ __forceinline__ uint32_t lower_bound(const uint32_t* __restrict__ ci, uint32_t b, uint32_t e, uint32_t x)
@@ -249,11 +248,12 @@ __global__ void __launch_bounds__(kThreads, 8) k_cc_init(const uint32_t* __restr
         row_range(rp, v, nnz, b, e);
         if ((v & 31u) == 0) {  // the tile's entries
             const uint32_t end = min(max(rp[min(i + 32, (uint64_t)n)], b), nnz);
-            if (end - b > kUnit) {
+            if (end - b > kBigTile) {
                 const unsigned long long units = (end - b - 1) / kUnit + 1;
                 const unsigned long long old = atomicAdd(big.head, 1ull << 32 | units);
                 if ((uint32_t)(old >> 32) < big.cap)  // (bad row pointers may list more)
                     big.list[old >> 32] = make_uint2(v / 32u, (uint32_t)old);
+                flags |= kFlagBig;
             }
         }
         uint32_t p = v;
@@ -287,24 +287,16 @@ __global__ void __launch_bounds__(kThreads) k_cc_flatten(uint32_t n, uint32_t* p
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_cc_hook(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
-                                                      uint32_t n, uint32_t nnz, uint32_t* parent, uint32_t* counters,
-                                                      BigTiles big)
+// (PART 0: every tile, 1: all but the big ones, 2: the units)
+template <int PART>
+__device__ __forceinline__ void hook_entries(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
+                                             uint32_t n, uint32_t nnz, uint32_t* parent, uint32_t* counters,
+                                             const BigTiles& big, uint2* list)
 {
     constexpr int U = kInFlight;
-    if (__ldcg(counters + 2) & kFlagRange)
-        return;  // bad row pointers (k_cc_init): the tiles need not partition the entries
     const uint32_t lane = threadIdx.x & 31u;
-    __shared__ uint2 pair_list[kThreads / 32][32 * U];
-    uint2* const list = pair_list[threadIdx.x >> 5];
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    const Work work(big);
     uint32_t flags = 0, lower = 0;
-    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < work.items; w += nwarps) {
-        uint32_t unit, kb, ke;
-        const uint32_t v0 = work.row_of(w, unit);
-        const RowTile t(rp, n, nnz, v0);
-        work.entries(w, unit, t, kb, ke);
+    auto visit = [&](uint32_t v0, const RowTile& t, uint32_t kb, uint32_t ke) {
         for (EntrySteps<U> es(kb, ke); es.more(); es.next()) {
             uint32_t v[U], u[U], ub[U], ue[U];
 #pragma unroll
@@ -393,13 +385,40 @@ __global__ void __launch_bounds__(kThreads) k_cc_hook(const uint32_t* __restrict
             }
             __syncwarp();
         }
-    }
+    };
+    if (PART == 2)
+        for_units(rp, n, nnz, big, visit);
+    else
+        for_tiles<PART == 1>(rp, n, nnz, visit);
     flags = __reduce_or_sync(0xFFFFFFFFu, flags);
     lower = __reduce_add_sync(0xFFFFFFFFu, lower);
     if (lane == 0 && flags)
         atomicOr(counters + 2, flags);
     if (lane == 0 && lower)
         atomicAdd(counters + 3, lower);
+}
+
+__device__ __noinline__ void hook_units(const uint32_t* rp, const uint32_t* ci, uint32_t n, uint32_t nnz,
+                                        uint32_t* parent, uint32_t* counters, BigTiles big, uint2* list)
+{
+    hook_entries<2>(rp, ci, n, nnz, parent, counters, big, list);
+}
+
+template <bool BIG>
+__global__ void __launch_bounds__(kThreads, BIG ? 4 : 0) k_cc_hook(const uint32_t* __restrict__ rp,
+                                                                   const uint32_t* __restrict__ ci, uint32_t n,
+                                                                   uint32_t nnz, uint32_t* parent, uint32_t* counters,
+                                                                   BigTiles big)
+{
+    // bad row pointers (k_cc_init): the tiles need not partition the entries; or big
+    // tiles, for the other form of this pass
+    if (__ldcg(counters + 2) & (BIG ? kFlagRange : kFlagRange | kFlagBig))
+        return;
+    __shared__ uint2 pair_list[kThreads / 32][32 * kInFlight];
+    uint2* const list = pair_list[threadIdx.x >> 5];
+    hook_entries<BIG ? 1 : 0>(rp, ci, n, nnz, parent, counters, big, list);
+    if (BIG)
+        hook_units(rp, ci, n, nnz, parent, counters, big, list);
 }
 
 // out_rp[v + 1] = length of row v + its links; counters[1] = number of links.
@@ -428,7 +447,8 @@ __global__ void __launch_bounds__(kThreads) k_connect_rowlen(const uint32_t* __r
 // column); a link e_j goes to out_rp[v] + (entries of v below e_j) + j.
 // Links never coincide with an entry (they join different components).
 // Writes past `cap` are dropped (the host reports the size needed).
-__global__ void __launch_bounds__(kThreads, 6) k_connect_copy(const uint32_t* __restrict__ rp,
+template <bool BIG>
+__global__ void __launch_bounds__(kThreads) k_connect_copy(const uint32_t* __restrict__ rp,
                                                            const uint32_t* __restrict__ ci, uint32_t n, uint32_t nnz,
                                                            const uint32_t* __restrict__ parent,
                                                            const uint32_t* counters, const uint32_t* __restrict__ out_rp,
@@ -439,13 +459,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_connect_copy(const uint32_t* __
         return;  // the call fails
     const uint32_t minn = __ldcg(counters);
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    const Work work(big);
-    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < work.items; w += nwarps) {
-        uint32_t unit, kb, ke;
-        const uint32_t v0 = work.row_of(w, unit);
-        const RowTile t(rp, n, nnz, v0);
-        work.entries(w, unit, t, kb, ke);
+    auto visit = [&](uint32_t v0, const RowTile& t, uint32_t kb, uint32_t ke) {
         uint32_t ob = 0, lk[2] = {0, 0};
         int nl = 0;
         if (v0 + (uint64_t)lane < n) {
@@ -478,44 +492,80 @@ __global__ void __launch_bounds__(kThreads, 6) k_connect_copy(const uint32_t* __
                     out_ci[at] = c[i];
             }
         }
-        for (int j = 0; j < nl && w < work.tiles; ++j) {
+        for (int j = 0; kb == t.beg && j < nl; ++j) {
             const uint64_t at = (uint64_t)ob + (lower_bound(ci, t.b, t.e, lk[j]) - t.b) + j;
             if (at < cap)
                 out_ci[at] = lk[j];
         }
-    }
+    };
+    for_tiles<BIG>(rp, n, nnz, visit);
+    if (BIG)
+        for_units(rp, n, nnz, big, visit);
+}
+
+int row_blocks(uint32_t n, int sms)
+{
+    return (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n + kThreads - 1) / kThreads, (uint64_t)sms * 8));
+}
+
+BigTiles big_tiles(uint2* list, uint32_t n, uint32_t* counters)
+{
+    return BigTiles{list, connect_tiles_cap(n), reinterpret_cast<unsigned long long*>(counters + 4)};
 }
 
 }  // namespace
 
 uint32_t connect_tiles_cap(uint32_t n) { return (uint32_t)(((uint64_t)n + 31) / 32); }
 
+namespace {
+
+// the unions of the entries and the passes behind them
+template <bool BIG>
+cudaError_t launch_entries(const uint32_t* rp, const uint32_t* ci, uint32_t n, uint32_t nnz, uint32_t* out_rp,
+                           uint32_t* out_ci, uint64_t cap, uint32_t* parent, uint32_t* partials, uint32_t* counters,
+                           const BigTiles& big, int sms, cudaStream_t st)
+{
+    // a warp per 32 rows, or per unit of a big tile
+    const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n + kThreads - 1) / kThreads +
+                                                                         (BIG ? nnz / (kUnit * (kThreads / 32)) : 0),
+                                                                     (uint64_t)sms * 16));
+    if (nnz > 0)
+        k_cc_hook<BIG><<<blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters, big);
+    k_connect_rowlen<<<row_blocks(n, sms), kThreads, 0, st>>>(rp, n, nnz, parent, counters, out_rp);
+    const cudaError_t e = launch_scan(out_rp + 1, n, partials, st);
+    if (e != cudaSuccess)
+        return e;
+    k_connect_copy<BIG><<<blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters, out_rp, out_ci, cap, big);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
 cudaError_t launch_connect(const uint32_t* rp, const uint32_t* ci, uint32_t n, uint32_t nnz, uint32_t* out_rp,
                            uint32_t* out_ci, uint64_t cap, uint32_t* parent, uint32_t* partials, uint32_t* counters,
                            uint2* tiles, int sms, cudaStream_t st)
 {
-    const int rows_blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n + kThreads - 1) / kThreads,
-                                                                          (uint64_t)sms * 8));
-    // the passes over entries: a warp per 32 rows, or per unit of a big tile
-    const int tile_blocks = (int)std::max<uint64_t>(
-        1, std::min<uint64_t>(((uint64_t)n + kThreads - 1) / kThreads + nnz / (kUnit * (kThreads / 32)),
-                              (uint64_t)sms * 16));
-    const BigTiles big{tiles, connect_tiles_cap(n), reinterpret_cast<unsigned long long*>(counters + 4)};
+    const BigTiles big = big_tiles(tiles, n, counters);
     cudaError_t e = cudaMemsetAsync(counters, 0xFF, sizeof(uint32_t), st);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(counters + 1, 0, 5 * sizeof(uint32_t), st);
     if (e != cudaSuccess)
         return e;
-    k_cc_init<<<rows_blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters, big);
-    k_cc_flatten<<<rows_blocks, kThreads, 0, st>>>(n, parent);
-    if (nnz > 0)
-        k_cc_hook<<<tile_blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters, big);
-    k_connect_rowlen<<<rows_blocks, kThreads, 0, st>>>(rp, n, nnz, parent, counters, out_rp);
-    e = launch_scan(out_rp + 1, n, partials, st);
+    k_cc_init<<<row_blocks(n, sms), kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters, big);
+    k_cc_flatten<<<row_blocks(n, sms), kThreads, 0, st>>>(n, parent);
+    return launch_entries<false>(rp, ci, n, nnz, out_rp, out_ci, cap, parent, partials, counters, big, sms, st);
+}
+
+cudaError_t launch_connect_big(const uint32_t* rp, const uint32_t* ci, uint32_t n, uint32_t nnz, uint32_t* out_rp,
+                               uint32_t* out_ci, uint64_t cap, uint32_t* parent, uint32_t* partials,
+                               uint32_t* counters, uint2* tiles, int sms, cudaStream_t st)
+{
+    // (links were counted before any union)
+    const cudaError_t e = cudaMemsetAsync(counters + 1, 0, 2 * sizeof(uint32_t), st);
     if (e != cudaSuccess)
         return e;
-    k_connect_copy<<<tile_blocks, kThreads, 0, st>>>(rp, ci, n, nnz, parent, counters, out_rp, out_ci, cap, big);
-    return cudaGetLastError();
+    return launch_entries<true>(rp, ci, n, nnz, out_rp, out_ci, cap, parent, partials, counters,
+                                big_tiles(tiles, n, counters), sms, st);
 }
 
 }  // namespace pbrcm

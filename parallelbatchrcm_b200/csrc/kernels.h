@@ -121,13 +121,19 @@ cudaError_t launch_scan(uint32_t* data, uint64_t m, uint32_t* partials, cudaStre
 // Workspace: parent (n), partials (scan_partials_count(n)), tiles
 // (connect_tiles_cap(n)), counters (6, 8-byte aligned):
 // [0] first non-empty row, [1] links added, [2] check flags (1 column out of
-// range or bad row pointers, 2 row not sorted, 4 not symmetric, 8 union limit),
-// [3] distinct entries below the diagonal less those above it (not 0: not
-// symmetric), [4..5] the head of `tiles`.
+// range or bad row pointers, 2 row not sorted, 4 not symmetric, 8 union limit,
+// kConnectBig), [3] distinct entries below the diagonal less those above it (not
+// 0: not symmetric), [4..5] the head of `tiles`.  kConnectBig alone: 32
+// consecutive rows somewhere have more than 1,024 entries, listed in `tiles`, and
+// nothing is joined yet: launch_connect_big does the rest (then read [1..3] again).
+constexpr uint32_t kConnectBig = 16;
 uint32_t connect_tiles_cap(uint32_t n);
 cudaError_t launch_connect(const uint32_t* rp, const uint32_t* ci, uint32_t n, uint32_t nnz, uint32_t* out_rp,
                            uint32_t* out_ci, uint64_t cap, uint32_t* parent, uint32_t* partials, uint32_t* counters,
                            uint2* tiles, int sms, cudaStream_t st);
+cudaError_t launch_connect_big(const uint32_t* rp, const uint32_t* ci, uint32_t n, uint32_t nnz, uint32_t* out_rp,
+                                 uint32_t* out_ci, uint64_t cap, uint32_t* parent, uint32_t* partials,
+                                 uint32_t* counters, uint2* tiles, int sms, cudaStream_t st);
 uint32_t permute_long_cap(uint32_t n, uint64_t nnz);
 constexpr uint32_t kPermuteWarpRow = 1024;  // longest row of the warp path
 cudaError_t launch_bandwidth(const uint32_t* rp, const uint32_t* ci, uint32_t n, const uint32_t* perm, uint32_t* inv,

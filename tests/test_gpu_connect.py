@@ -167,11 +167,11 @@ def _hubs_apart(sizes, at, seed):
     return rp, c[o].astype(np.uint32)
 
 
-@pytest.mark.parametrize("sizes", [[993], [992], [994], [1024], [1025], [1026], [2018, 2], [2048], [5000],
+@pytest.mark.parametrize("sizes", [[992], [993], [994], [1024], [1025], [1026], [1504, 2], [1536], [20000],
                                    [700, 700, 700, 3000, 50], [1100] * 70])
 @pytest.mark.parametrize("at", [0, 31, 500])
 def test_long_rows(pbrcm, gpu_ctx, oracle_mod, sizes, at):
-    """Groups of 32 rows around the 1,024 entries a warp takes at a time and
+    """Groups of 32 rows around the 1,024 entries up to which a warp takes them and
     far beyond, one and many, with links falling into them."""
     _check(pbrcm, gpu_ctx, oracle_mod, *_hubs_apart(sizes, at, len(sizes) + at))
 
@@ -197,3 +197,17 @@ def test_hub_row_is_shared_out(pbrcm, gpu_ctx):
             best[name] = min(best.get(name, 1e9), time.perf_counter() - t)
         assert links == 0
     assert best["star"] < 10 * best["path"], best
+
+
+def test_long_rows_one_sided(pbrcm, gpu_ctx):
+    """An entry without its transpose in a long row, and in a short one beside
+    long rows, is still refused."""
+    rp, ci = _hubs_apart([5000], 31, 3)
+    n = rp.size - 1
+    rows = [ci[rp[r]:rp[r + 1]] for r in range(n)]
+    single = next(r for r in range(n) if rows[r].size == 1 and r > 40)
+    for r, c in ((31, single), (single, 31), (single, single - 1)):
+        bad = [np.union1d(x, [c]).astype(np.uint32) if i == r else x for i, x in enumerate(rows)]
+        brp = np.concatenate([[0], np.cumsum([x.size for x in bad])]).astype(np.uint32)
+        with pytest.raises(pbrcm.PbrcmError):
+            _run(pbrcm, gpu_ctx, brp, np.concatenate(bad))
